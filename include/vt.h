@@ -191,9 +191,9 @@ typedef struct {
     int record_trace;      /* log per-frame touched coarse nodes */
     int trace_level;       /* octree level of the logged nodes (4 in C4) */
     int record_hits;       /* keep per-ray hit node/brick/t/normal for vt_debug_hits */
-    int persistent;        /* 1: persistent ray-queue kernel with warp refill */
-    int blocks_per_sm;     /* persistent grid: CTAs per SM (autotuned) */
-    int pops;              /* persistent: traversal steps between warp refills */
+    /* accepted and kept, without effect on the trace kernel, which has one
+     * schedule (blocks_per_sm still sizes the wavefront passes' grid) */
+    int persistent, blocks_per_sm, pops;
     int preload;           /* 1: load every needed brick at create when they fit */
     int use_graph;         /* 1: pass 0 of a frame replays a captured CUDA graph */
     int refine;            /* isovalue crossing refinement: 0 = one linear step, as the
@@ -261,8 +261,7 @@ vt_status vt_change_num_rays(vt_handle* h, int numRayPx);
 vt_status vt_change_cache(vt_handle* h, int maxElements, const int cubeDim[3], int cubeInc);
 
 /* Kernel schedule knobs of a live handle (autotuner): ray-tile shape,
- * march unroll, persistent ray queue, traversal steps between refills,
- * persistent CTAs per SM, lookahead requests, graph replay, absent-brick
+ * march unroll, lookahead requests, graph replay, absent-brick
  * candidates set aside per pass, side-stream lookahead loads, wavefront
  * rounds, shared aprons, demand batch. */
 typedef struct {
@@ -279,7 +278,7 @@ vt_status vt_render(vt_handle* h, float* dev_rgba, uint8_t* dev_rgb8, void* stre
 /* Same with host output buffers (copies included); synchronises. */
 vt_status vt_render_host(vt_handle* h, float* host_rgba, uint8_t* host_rgb8);
 
-/* Many views in one persistent ray-queue launch (no reference counterpart). */
+/* Many views in one launch (no reference counterpart). */
 typedef struct {
     vt_camera cam;
     float* dev_rgba;        /* W*H*4 floats, may be NULL if dev_rgb8 given */

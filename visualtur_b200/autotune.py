@@ -1,10 +1,10 @@
 """Autotuner for the ray-casting kernels (no reference counterpart).
 
 Sweeps the kernel schedule of a live renderer -- ray-tile size {32, 64,
-128, 256 rays}, march unroll {1, 2, 4, 8}, one-ray-per-thread vs the
-persistent ray queue and the queue's refill interval {8, ..., 128 steps}
--- and, through a caller-supplied factory, the brick
-size {8, 16, 32} (which needs a new renderer: the cache layout changes).
+128, 256 rays} and march unroll {1, 2, 4, 8} -- and, through a
+caller-supplied factory, the brick size {8, 16, 32} (which needs a new
+renderer: the cache layout changes).  The persistent and pops knobs can
+still be swept; the trace kernel has one schedule whatever they say.
 Each point is timed with CUDA events over the same frames after a warm-up
 that leaves the brick cache in the same state; the fastest is kept.
 """
@@ -12,8 +12,8 @@ import itertools
 
 TILES = {32: (8, 4), 64: (8, 8), 128: (16, 8), 256: (16, 16)}
 UNROLLS = (1, 2, 4, 8)
-PERSIST = (0, 1)
-POPS = (8, 16, 32, 64, 128)       # persistent queue: traversal steps between warp refills
+PERSIST = (0,)
+POPS = ()
 
 
 def time_frames(torch, renderer, render_step, frames, warmup=2, stream=None):
@@ -35,8 +35,8 @@ def time_frames(torch, renderer, render_step, frames, warmup=2, stream=None):
 
 def tune_schedule(torch, renderer, render_step, frames=6, tiles=TILES, unrolls=UNROLLS, persist=PERSIST,
                   stream=None, pops=POPS):
-    """Best (tile, unroll, persistent) for a renderer, then -- when the
-    persistent queue wins -- its refill interval; returns (best, table)."""
+    """Best (tile, unroll, persistent) for a renderer and, where `pops` names
+    any, the best of them with persistent set; returns (best, table)."""
     table = []
     for (rays, (tw, th)), u, p in itertools.product(sorted(tiles.items()), unrolls, persist):
         renderer.set_tuning(tile_w=tw, tile_h=th, unroll=u, persistent=p)
@@ -47,7 +47,6 @@ def tune_schedule(torch, renderer, render_step, frames=6, tiles=TILES, unrolls=U
     renderer.set_tuning(tile_w=best["tile_w"], tile_h=best["tile_h"], unroll=best["unroll"],
                         persistent=best["persistent"])
     if best["persistent"] and pops:
-        # second stage: refill interval of the persistent queue at the best shape
         for pp in pops:
             renderer.set_tuning(pops=pp)
             ms = time_frames(torch, renderer, render_step, frames, stream=stream)

@@ -14,8 +14,8 @@
  * in DFS order still decides the pixel.
  *
  * Octree: a flattened node array with 8-bit child masks holding the result
- * of the reference's range search (computed once per octree load), so a
- * traversal step is 8 slab tests and a popcount instead of binary searches.
+ * of the reference's range search (computed once per octree load), and the
+ * same tree two levels at a time (tree64.cuh), which k_trace walks.
  */
 #include "vt_kernels.h"
 #include "vt_math.cuh"
@@ -116,66 +116,73 @@ __device__ __forceinline__ float3 normal_at(const Samp& s, float3 p) {
 }
 
 /* The march of cuda_rayCaster (src/rayCaster.cu:166-237): samples at
- * Xnear, Xnear += 0.5*dir, for steps 0..maxStep; the first sign change of
- * iso - value (equality counts) is refined once linearly.  U samples are
- * fetched per round: their positions accumulate in the reference's order,
- * their taps are issued together, and the crossing test then runs sample
- * by sample -- fetches past the hit are discarded (indices stay clamped to
- * the brick) and are not counted.
- *
- * refine > 0 bisects the bracketing pair [previous, current sample] that
- * many times before the linear step: the midpoint replaces the end whose
- * iso - value has the same strict sign as its own (the crossing test's
- * "no crossing" condition), so the pair keeps bracketing the crossing.
- * Each midpoint is one more trilinear sample. */
+ * Xnear, Xnear += 0.5*dir, for steps 0..maxStep, to the first sign change of
+ * iso - value (equality counts).  U samples are fetched per round: their
+ * positions accumulate in the reference's order, their taps are issued
+ * together, and the crossing test then runs sample by sample -- fetches
+ * past the crossing are discarded (indices stay clamped to the brick) and
+ * are not counted.  A crossing leaves the sample before it in C. */
+struct Crossing {
+    float3 P;        /* last sample before the crossing; the crossing sample is P + 0.5*dir */
+    float ant, sig;  /* their values */
+};
 template <int VTYPE, bool SLAB, int U, bool SHM = false>
-__device__ __forceinline__ bool march(const Samp& s, float3 origin, float3 ray, float tnear,
-                                      int maxStep, float iso, int refine, float3* Xhit, unsigned int* nsamp) {
-    float3 Xnear = add(origin, mul(ray, tnear));
-    float3 Xfar = Xnear;
-    float3 vStep = mul(ray, 0.5f);
+__device__ __forceinline__ bool march(const Samp& s, float3 origin, float3 ray, float tnear, int maxStep, float iso,
+                                      Crossing& C, unsigned int* nsamp) {
+    const float3 vStep = mul(ray, 0.5f);
     if (maxStep < 0) return false;
-    float ant = interp<VTYPE, SLAB, SHM>(s, Xnear);
+    C.P = add(origin, mul(ray, tnear));
+    C.ant = interp<VTYPE, SLAB, SHM>(s, C.P);
     unsigned int ns = 1;
     bool hit = false;
     for (int steps = 1; steps <= maxStep && !hit; steps += U) {
         float3 X[U];
         float v[U];
 #pragma unroll
-        for (int u = 0; u < U; u++) X[u] = add(u == 0 ? Xnear : X[u - 1], vStep);
+        for (int u = 0; u < U; u++) X[u] = add(u == 0 ? C.P : X[u - 1], vStep);
 #pragma unroll
         for (int u = 0; u < U; u++) v[u] = interp<VTYPE, SLAB, SHM>(s, X[u]);
 #pragma unroll
         for (int u = 0; u < U; u++) {
             if (hit || steps + u > maxStep) break;
-            float sig = v[u];
+            C.sig = v[u];
             ns++;
-            if ((((iso - ant) < 0.0f) && ((iso - sig) < 0.0f)) ||
-                (((iso - ant) > 0.0f) && ((iso - sig) > 0.0f))) {
-                ant = sig;
-                Xfar = X[u];
+            if ((((iso - C.ant) < 0.0f) && ((iso - C.sig) < 0.0f)) ||
+                (((iso - C.ant) > 0.0f) && ((iso - C.sig) > 0.0f))) {
+                C.ant = C.sig;
+                C.P = X[u];
             } else {
-                float3 P = Xfar, Q = X[u];
-                for (int k = 0; k < refine; k++) {
-                    float3 M = mul(add(P, Q), 0.5f);
-                    float vm = interp<VTYPE, SLAB, SHM>(s, M);
-                    ns++;
-                    if ((((iso - ant) < 0.0f) && ((iso - vm) < 0.0f)) ||
-                        (((iso - ant) > 0.0f) && ((iso - vm) > 0.0f))) {
-                        P = M; ant = vm;
-                    } else {
-                        Q = M; sig = vm;
-                    }
-                }
-                float a = (iso - ant) / (sig - ant);
-                *Xhit = add(mul(P, 1.0f - a), mul(Q, a));
                 hit = true;
             }
         }
-        Xnear = X[U - 1];
     }
     *nsamp += ns;
     return hit;
+}
+
+/* The crossing refined to the hit point (src/rayCaster.cu:227-228): one
+ * linear step.  refine > 0 first bisects the bracketing pair that many
+ * times: the midpoint replaces the end whose iso - value has the same
+ * strict sign as its own (the crossing test's "no crossing" condition), so
+ * the pair keeps bracketing the crossing.  Each midpoint is one more
+ * trilinear sample. */
+template <int VTYPE, bool SLAB, bool SHM>
+__device__ __forceinline__ float3 refine_hit(const Samp& s, float3 ray, const Crossing& C, float iso, int refine,
+                                             unsigned int* nsamp) {
+    float3 P = C.P, Q = add(C.P, mul(ray, 0.5f));
+    float ant = C.ant, sig = C.sig;
+    for (int k = 0; k < refine; k++) {
+        float3 M = mul(add(P, Q), 0.5f);
+        float vm = interp<VTYPE, SLAB, SHM>(s, M);
+        if ((((iso - ant) < 0.0f) && ((iso - vm) < 0.0f)) || (((iso - ant) > 0.0f) && ((iso - vm) > 0.0f))) {
+            P = M; ant = vm;
+        } else {
+            Q = M; sig = vm;
+        }
+    }
+    *nsamp += refine;
+    float a = (iso - ant) / (sig - ant);
+    return add(mul(P, 1.0f - a), mul(Q, a));
 }
 
 /* Stack entry: (node index in its level << code_bits) | Morton code. */
@@ -196,26 +203,22 @@ __device__ __forceinline__ unsigned int e_x(unsigned long long e) { return (unsi
 __device__ __forceinline__ unsigned int e_y(unsigned long long e) { return (unsigned int)(e >> VT_E_COORD_BITS) & 0x7FFu; }
 __device__ __forceinline__ unsigned int e_z(unsigned long long e) { return (unsigned int)e & 0x7FFu; }
 
-/* sampler for the brick at brick coordinates (bx,by,bz) */
+/* sampler for the brick at brick coordinates (bx,by,bz), in device slot `slot` */
 template <int VTYPE, bool SLAB>
-__device__ __forceinline__ void setup_sampler(const TraceArgs& A, unsigned int bx, unsigned int by, unsigned int bz,
-                                              unsigned int pidx, Samp& s, int* slot) {
+__device__ __forceinline__ void brick_sampler(const TraceArgs& A, unsigned int bx, unsigned int by, unsigned int bz,
+                                              int slot, Samp& s) {
     const DevBricks& B = A.br;
     if (SLAB) {
         const int sh = A.oct.nLevels - A.oct.Lc;
         s.ox = (float)((int)(bx << sh) - B.inc); s.oy = (float)((int)(by << sh) - B.inc);
         s.oz = (float)((int)(bz << sh) - B.inc);
-        int sl = B.page[pidx];
-        *slot = sl;
-        if (sl < 0) return;
-        s.base = (const char*)B.slab + (size_t)sl * (size_t)B.brickVol * (VTYPE == 0 ? 4 : 1);
+        s.base = (const char*)B.slab + (size_t)slot * (size_t)B.brickVol * (VTYPE == 0 ? 4 : 1);
         s.sx = B.D * B.D; s.sy = B.D;
         s.h = (float)(B.D - 2);
     } else {
         /* dense: index space = the padded volume, global voxel g at g + P.
          * Equals the brick-relative index of the reference whenever every
          * tap lies inside the brick and its apron (cubeInc >= 3). */
-        *slot = 0;
         s.ox = s.oy = s.oz = (float)-B.P;
         s.base = B.vol;
         s.sx = (int)B.vsx; s.sy = (int)B.vsy;
@@ -239,6 +242,7 @@ struct Ray {
     int nskip;             /* candidates passed over (brick absent), in st.sk */
     bool tent;             /* the pixel holds a hit found past them */
     bool resumeSkips;      /* the passed-over candidates come first (a resumed ray) */
+    unsigned int taken;    /* candidates the 64-ary walk has already dealt with */
 };
 
 /* RAY_TENTATIVE: a hit past passed-over candidates (the pixel is written,
@@ -441,8 +445,7 @@ __device__ __forceinline__ int candidate(const TraceArgs& A, Ray& R, unsigned lo
     const unsigned int x = e_x(ent), y = e_y(ent), z = e_z(ent);
     const unsigned int bx = x >> (Lo - Lc), by = y >> (Lo - Lc), bz = z >> (Lo - Lc);
     const unsigned int pidx = (bx << (2 * Lc)) | (by << Lc) | bz;
-    Samp s; int slot;
-    setup_sampler<VTYPE, SLAB>(A, bx, by, bz, pidx, s, &slot);
+    const int slot = SLAB ? A.br.page[pidx] : 0;
     if (SLAB && slot < 0) {
         if (slot == -1 || slot == VT_PAGE_SPECULATIVE) request_brick(A, pidx);
         cnt[VT_C_DEVMISSES]++;
@@ -461,11 +464,12 @@ __device__ __forceinline__ int candidate(const TraceArgs& A, Ray& R, unsigned lo
     const int mbx = (int)(x << (nLevels - Lo)), mby = (int)(y << (nLevels - Lo)), mbz = (int)(z << (nLevels - Lo));
     float tn, tf;
     if (!slab(R.r, mbx, mby, mbz, mbx + dimO, mby + dimO, mbz + dimO, &tn, &tf)) return CAND_EMPTY;
-    float3 X;
-    unsigned int ns = 0;
-    bool h = march<VTYPE, SLAB, U>(s, R.r.o, R.dir, tn, max_steps(tn, tf), A.iso, A.refine, &X, &ns);
-    cnt[VT_C_SAMPLES] += ns;
-    if (!h) return CAND_EMPTY;
+    Samp s;
+    brick_sampler<VTYPE, SLAB>(A, bx, by, bz, slot, s);
+    Crossing C;
+    if (!march<VTYPE, SLAB, U>(s, R.r.o, R.dir, tn, max_steps(tn, tf), A.iso, C, &cnt[VT_C_SAMPLES]))
+        return CAND_EMPTY;
+    const float3 X = refine_hit<VTYPE, SLAB, false>(s, R.dir, C, A.iso, A.refine, &cnt[VT_C_SAMPLES]);
     shade_hit<VTYPE, SLAB, false>(A, R, s, X, x, y, z, bx, by, bz, cnt);
     return CAND_HIT;
 }
@@ -516,6 +520,7 @@ __device__ int run_ray(const TraceArgs& A, Ray& R, Stk& st, unsigned int* cnt, i
             if (!expand(A, R.r, st, R.top, ent, cnt, true)) return RAY_DONE;
         }
         if (budget-- == 0) return RAY_RUNNING;
+        if (R.taken) { R.taken--; R.top--; continue; }
         const int c = candidate<VTYPE, SLAB, U>(A, R, ent, cnt);
         if (c == CAND_MISSING) {
             if (SKIP && R.nskip < K) { st.sk[R.nskip++] = ent; R.top--; continue; }
@@ -558,7 +563,8 @@ __device__ void lookahead_requests(const TraceArgs& A, Ray R, Stk& st, unsigned 
 __device__ __forceinline__ bool decode_ray(const DevView* sv, int nv, int tw, int th, unsigned int g, int& v, int& i,
                                            int& j) {
     v = 0;
-    for (int k = 1; k < nv; k++) if (sv[k].rayBase <= g) v = k;
+    for (int b = VT_MAX_VIEWS / 2; b; b >>= 1)   /* last view whose base is <= g */
+        if (v + b < nv && sv[v + b].rayBase <= g) v += b;
     unsigned int local = g - sv[v].rayBase;
     unsigned int tile = local / (unsigned)(tw * th), lt = local % (unsigned)(tw * th);
     unsigned int ti = tile / sv[v].tilesX, tj = tile % sv[v].tilesX;
@@ -567,44 +573,45 @@ __device__ __forceinline__ bool decode_ray(const DevView* sv, int nv, int tw, in
     return i < sv[v].cam.H && j < sv[v].cam.W;
 }
 
-/* Sets up work item w (pass 0: padded ray index; later passes: suspended
- * record).  Returns RAY_RUNNING when the ray has traversal to do, RAY_DONE
- * when it is background already (root miss), -1 for tile padding. */
-template <int VTYPE, bool SKIP>
-__device__ int start_ray(const TraceArgs& A, const DevView* sv, unsigned int w, Ray& R, Stk& st,
-                          unsigned int* cnt) {
-    unsigned int depth = 0;
-    unsigned long long off = 0;
-    bool resume = A.ctl.in != nullptr;
-    if (resume) {
-        SuspRec rec = A.ctl.in[w];
-        R.g = rec.ray; depth = rec.depth; off = rec.off;
-    } else {
-        R.g = w;
-    }
-    if (!decode_ray(sv, A.views.n, A.tile_w, A.tile_h, R.g, R.view, R.i, R.j)) return -1;
-    const DevCamera& C = sv[R.view].cam;
-    R.dir = ray_dir(C.look, C.up, C.right, C.dist, C.h, C.w, C.H, C.W, R.i, R.j);
-    R.r.o = C.pos; R.r.dx = 1 / R.dir.x; R.r.dy = 1 / R.dir.y; R.r.dz = 1 / R.dir.z;
+/* ray g's camera ray; false for tile padding */
+__device__ __forceinline__ bool ray_of(const TraceArgs& A, const DevView* sv, unsigned int g, int& view, int& i, int& j,
+                                       float3& dir, RayInv& r) {
+    if (!decode_ray(sv, A.views.n, A.tile_w, A.tile_h, g, view, i, j)) return false;
+    const DevCamera& C = sv[view].cam;
+    dir = ray_dir(C.look, C.up, C.right, C.dist, C.h, C.w, C.H, C.W, i, j);
+    r.o = C.pos; r.dx = 1 / dir.x; r.dy = 1 / dir.y; r.dz = 1 / dir.z;
+    return true;
+}
+
+/* Sets up ray rec.ray for the literal search: from the root (fresh rays,
+ * depth 0), from its saved stack, or, suspended by the 64-ary walk, from
+ * the root passing over the candidates it has taken.  Returns RAY_RUNNING
+ * when the ray has traversal to do, RAY_DONE when it is background already
+ * (root miss), -1 for tile padding. */
+template <bool SKIP>
+__device__ int start_ray(const TraceArgs& A, const DevView* sv, const SuspRec& rec, Ray& R, Stk& st) {
+    R.g = rec.ray;
+    if (!ray_of(A, sv, R.g, R.view, R.i, R.j, R.dir, R.r)) return -1;
     R.rgba = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
     R.hit = false; R.node = 0; R.brick = 0; R.t = -1.0f; R.n = f3(0, 0, 0);
     R.top = -1;
     R.lastSlot = -1;
-    R.nskip = 0; R.tent = false; R.resumeSkips = false;
-    if (resume && depth > 0) {
+    R.nskip = 0; R.tent = false; R.resumeSkips = false; R.taken = 0;
+    if (rec.depth & VT_SUSP_WALK) {
+        R.taken = rec.depth >> VT_SUSP_TAKEN_SHIFT;
+    } else if (rec.depth > 0) {
         int nsk = 0;
         if (SKIP) {
-            nsk = (int)((depth >> 8) & 7u);
+            nsk = (int)((rec.depth >> 8) & 7u);
             R.nskip = nsk;
-            R.tent = (depth >> 11) & 1u;
+            R.tent = (rec.depth >> 11) & 1u;
             R.resumeSkips = nsk > 0 || R.tent;
-            for (int e = 0; e < nsk; e++) st.sk[e] = A.ctl.pool_in[off + e];
+            for (int e = 0; e < nsk; e++) st.sk[e] = A.ctl.pool_in[rec.off + e];
         }
-        R.top = (int)(depth & 255u) - 1;
-        for (int e = 0; e <= R.top; e++) st.e[e] = A.ctl.pool_in[off + nsk + e];
+        R.top = (int)(rec.depth & 255u) - 1;
+        for (int e = 0; e <= R.top; e++) st.e[e] = A.ctl.pool_in[rec.off + nsk + e];
         return RAY_RUNNING;
     }
-    if (!resume) cnt[VT_C_RAYS]++;
     const int N = 1 << A.oct.nLevels;
     float tn, tf;
     /* root test (src/Octree.cu:729) */
@@ -669,70 +676,313 @@ __device__ __forceinline__ void flush_counters(const TraceArgs& A, unsigned int*
     }
 }
 
-/* One ray per thread (PERSIST = false) or a persistent ray queue: each warp
- * keeps its 32 lanes busy, and after every `pops` traversal steps the lanes
- * whose ray finished or suspended take new work items -- a ballot of the
- * idle lanes, one atomicAdd by the leader, and a popcount rank per lane.
- * Eight 128-thread CTAs per SM (64 registers a thread): the traversal is
- * latency-bound, and the extra resident warps hide more of it than the
- * few spilled registers cost. */
-template <int VTYPE, bool SLAB, bool PERSIST, int U, bool SKIP>
-__global__ void __launch_bounds__(128, 8) k_trace(TraceArgs A) {
-    __shared__ DevView sv[VT_MAX_VIEWS];
-    for (int k = threadIdx.x; k < A.views.n; k += blockDim.x) sv[k] = A.views.v[k];
+/* The literal depth-first search for one ray, to its end: rays whose 64-ary
+ * walk met coinciding or non-finite plane products, and rays resumed with a
+ * saved stack (a wavefront round's).  Rare, so it is kept out of line: its
+ * stack and its registers cost the others nothing.  sk: set-aside
+ * candidates of a ray handed over by the walk. */
+template <int VTYPE, bool SLAB, int U, bool SKIP>
+__device__ __noinline__ void literal_ray(const TraceArgs& A, const DevView* sv, SuspRec rec, int nskip,
+                                         const unsigned long long* sk) {
+    unsigned int cnt[VT_C_COUNT];
+    for (int c = 0; c < VT_C_COUNT; c++) cnt[c] = 0;
+    Stk st;
+    Ray R;
+    int s = start_ray<SKIP>(A, sv, rec, R, st);
+    if (s < 0) return;
+    if (SKIP && nskip > 0) {
+        R.nskip = nskip;
+        for (int e = 0; e < nskip; e++) st.sk[e] = sk[e];
+    }
+    if (s == RAY_RUNNING) s = run_ray<VTYPE, SLAB, U, SKIP>(A, R, st, cnt, -1);
+    if (s == RAY_DONE) write_ray(A, sv, R, cnt);
+    else if (SKIP && s == RAY_TENTATIVE) {
+        write_ray(A, sv, R, cnt, false);
+        suspend_ray<VTYPE, SLAB, SKIP>(A, R, st, cnt);
+    } else if (s == RAY_SUSPENDED) suspend_ray<VTYPE, SLAB, SKIP>(A, R, st, cnt);
+    else if (SKIP && s == RAY_DONE_WRITTEN) cnt[VT_C_HITS]++;   /* the tentative hit stands */
+    for (int c = 0; c < VT_C_COUNT; c++) {
+        if (!cnt[c]) continue;
+        if (c == VT_C_MAXSTACK) atomicMax(&A.ctl.counters[c], (unsigned long long)cnt[c]);
+        else atomicAdd(&A.ctl.counters[c], (unsigned long long)cnt[c]);
+    }
+}
+
+#define VT_TRACE_THREADS 128
+#define VT_TRACE_CTAS 7
+
+/* One ray of k_trace in flight. */
+struct Trip {
+    RayInv r;
+    float3 dir;
+    Walk w;
+    int cx, cy, cz;            /* candidate last looked at */
+    unsigned int g;            /* padded global ray index */
+    int view, i, j;
+    bool fresh;                /* the walk's current cell is still to be looked at */
+    unsigned int taken;        /* candidates dealt with so far */
+    unsigned int pidx; int slot;   /* brick of the last resident candidate (its page cannot change in a pass) */
+    Crossing C;                /* a hit's crossing (refined and shaded when the ray is finished) */
+    /* set-aside candidates (SKIP) */
+    int nskip;
+    bool tent, resumeSkips;    /* as Ray's */
+    bool ended;                /* the walk is over; only set-aside candidates are left */
+};
+/* how a ray left the advance loop (besides RAY_*) */
+enum { TRIP_MISS = 5, TRIP_LITERAL = 6 };
+
+/* Candidate (R.cx, R.cy, R.cz), whose cell the ray crosses from product tn
+ * to tf: brick lookup (lruCache::updateCube, src/lruCache.cu:177-291) and
+ * march (src/rayCaster.cu:139-237).  CAND_MISSING when the brick is absent
+ * (it is requested), CAND_HIT with the crossing in R.C. */
+template <int VTYPE, bool SLAB, int U>
+__device__ __forceinline__ int try_candidate(const TraceArgs& A, Trip& R, float tn, float tf, unsigned int* cnt) {
+    const int Lo = A.oct.Lo, Lc = A.oct.Lc;
+    const unsigned int bx = (unsigned)R.cx >> (Lo - Lc), by = (unsigned)R.cy >> (Lo - Lc), bz = (unsigned)R.cz >> (Lo - Lc);
+    const unsigned int pidx = (bx << (2 * Lc)) | (by << Lc) | bz;
+    if (SLAB && pidx != R.pidx) {
+        const int slot = A.br.page[pidx];
+        if (slot < 0) {
+            if (slot == -1 || slot == VT_PAGE_SPECULATIVE) request_brick(A, pidx);
+            cnt[VT_C_DEVMISSES]++;
+            return CAND_MISSING;
+        }
+        R.pidx = pidx; R.slot = slot;
+        A.br.stamp[slot] = A.br.pass;
+    }
+    cnt[VT_C_CANDIDATES]++;
+    if (A.ctl.touched) {
+        const int d = A.ctl.touch_shift / 3;   /* Lo - trace level */
+        const unsigned long long n = (spread3((unsigned)R.cx >> d) << 2) | (spread3((unsigned)R.cy >> d) << 1) |
+                                     spread3((unsigned)R.cz >> d);
+        atomicOr(&A.ctl.touched[n >> 5], 1u << (n & 31));
+    }
+    Samp s;
+    brick_sampler<VTYPE, SLAB>(A, bx, by, bz, R.slot, s);
+    return march<VTYPE, SLAB, U>(s, R.r.o, R.dir, tn, max_steps(tn, tf), A.iso, R.C, &cnt[VT_C_SAMPLES]) ? CAND_HIT
+                                                                                                        : CAND_EMPTY;
+}
+
+/* Sets up ray rec.ray: RAY_RUNNING (walk to do), TRIP_MISS (background),
+ * TRIP_LITERAL, or -1 for tile padding. */
+template <bool SKIP>
+__device__ __forceinline__ int start_trip(const TraceArgs& A, const DevView* sv, const SuspRec& rec, Trip& R,
+                                          uint2* path, unsigned long long* sk) {
+    R.g = rec.ray;
+    R.pidx = 0xFFFFFFFFu; R.slot = 0;
+    R.fresh = true; R.taken = 0;
+    R.nskip = 0; R.tent = false; R.resumeSkips = false; R.ended = false;
+    if (rec.depth && !(rec.depth & VT_SUSP_WALK)) return TRIP_LITERAL;   /* a saved stack */
+    if (!ray_of(A, sv, R.g, R.view, R.i, R.j, R.dir, R.r)) return -1;
+    if (rec.depth) {
+        R.taken = rec.depth >> VT_SUSP_TAKEN_SHIFT;
+        int nsk = 0;
+        if (SKIP) {
+            nsk = (int)((rec.depth >> 8) & 7u);
+            R.nskip = nsk;
+            R.tent = (rec.depth >> 11) & 1u;
+            R.resumeSkips = nsk > 0 || R.tent;
+            for (int e = 0; e < nsk; e++) sk[e] = A.ctl.pool_in[rec.off + e];
+        }
+        if (rec.depth & 255u) {
+            const unsigned long long c = A.ctl.pool_in[rec.off + nsk];
+            walk_at<VT_TRACE_THREADS>(A.oct.t64, R.r, (int)e_x(c), (int)e_y(c), (int)e_z(c), R.w, path);
+        } else {
+            R.ended = true;
+        }
+        return RAY_RUNNING;
+    }
+    if (!A.oct.rootValid) return TRIP_MISS;
+    const int s = walk_root<VT_TRACE_THREADS>(A.oct.t64, R.r, R.w, path);
+    return s == WALK_CANDIDATE ? RAY_RUNNING : s == WALK_END ? TRIP_MISS : TRIP_LITERAL;
+}
+
+/* Takes a running ray to its end: walk to the next candidate, march it,
+ * until a hit, an absent brick or the end of the walk.  Set-aside candidates
+ * as in run_ray. */
+template <int VTYPE, bool SLAB, int U, bool SKIP>
+__device__ __forceinline__ int advance_trip(const TraceArgs& A, Trip& R, uint2* path, unsigned long long* sk,
+                                            unsigned int* cnt) {
+    if (SKIP) {
+        while (R.resumeSkips) {
+            if (R.nskip == 0) {
+                R.resumeSkips = false;
+                if (R.tent) return RAY_DONE_WRITTEN;
+                if (R.ended) return TRIP_MISS;
+                break;
+            }
+            R.cx = (int)e_x(sk[0]); R.cy = (int)e_y(sk[0]); R.cz = (int)e_z(sk[0]);
+            const int sh = A.oct.nLevels - A.oct.Lo;
+            float tn, tf;
+            slab(R.r, R.cx << sh, R.cy << sh, R.cz << sh, (R.cx + 1) << sh, (R.cy + 1) << sh, (R.cz + 1) << sh, &tn, &tf);
+            const int c = try_candidate<VTYPE, SLAB, U>(A, R, tn, tf, cnt);
+            if (c == CAND_MISSING) return RAY_SUSPENDED;
+            for (int k = 1; k < R.nskip; k++) sk[k - 1] = sk[k];
+            R.nskip--;
+            if (c == CAND_HIT) { R.nskip = 0; return RAY_DONE; }
+        }
+    }
+    const int K = SKIP ? A.ctl.skip : 0;
+    for (;;) {
+        int budget = 0x7FFFFFFF;
+        float tf;
+        const int s = walk_next<VT_TRACE_THREADS>(A.oct.t64, R.r, R.w, path, R.fresh, budget, &tf, &cnt[VT_C_EXPANSIONS]);
+        if (s == WALK_TIE) return TRIP_LITERAL;
+        if (s == WALK_END) {
+            if (SKIP && R.nskip > 0) { R.ended = true; return RAY_SUSPENDED; }
+            return TRIP_MISS;
+        }
+        walk_cell(A.oct.t64, R.r, R.w, R.cx, R.cy, R.cz);
+        const int c = try_candidate<VTYPE, SLAB, U>(A, R, R.w.tc < 0.0f ? 0.0f : R.w.tc, tf, cnt);
+        if (c == CAND_MISSING) {
+            if (!SKIP || R.nskip >= K) return RAY_SUSPENDED;   /* the candidate is the one to resume at */
+            sk[R.nskip++] = make_entry(0, A.oct.Lo, R.cx, R.cy, R.cz);
+        }
+        R.taken++;
+        R.fresh = false;
+        if (c == CAND_HIT) return (!SKIP || R.nskip == 0) ? (int)RAY_DONE : (int)RAY_TENTATIVE;
+    }
+}
+
+/* Speculative requests: walks on from a suspended ray's candidate (without
+ * marching) and requests up to `lookahead` further absent bricks. */
+__device__ __forceinline__ void lookahead_walk(const TraceArgs& A, Trip& R, uint2* path) {
+    const int Lo = A.oct.Lo, Lc = A.oct.Lc;
+    int want = A.ctl.lookahead, budget = 256;
+    unsigned int last = 0xFFFFFFFFu, entered = 0;
+    bool fresh = true;
+    while (want > 0 && budget-- > 0) {
+        float tf;
+        if (walk_next<VT_TRACE_THREADS>(A.oct.t64, R.r, R.w, path, fresh, budget, &tf, &entered) != WALK_CANDIDATE) break;
+        walk_cell(A.oct.t64, R.r, R.w, R.cx, R.cy, R.cz);
+        const unsigned int pidx = (((unsigned)R.cx >> (Lo - Lc)) << (2 * Lc)) | (((unsigned)R.cy >> (Lo - Lc)) << Lc) |
+                                  ((unsigned)R.cz >> (Lo - Lc));
+        if (pidx != last && A.br.page[pidx] == -1) { request_brick(A, pidx, true); want--; }
+        last = pidx;
+        fresh = false;
+    }
+}
+
+template <bool SLAB, bool SKIP>
+__device__ __forceinline__ void suspend_trip(const TraceArgs& A, Trip& R, uint2* path,
+                                             const unsigned long long* sk, unsigned int* cnt) {
+    cnt[VT_C_SUSPENDED]++;
+    unsigned int q = atomicAdd(A.ctl.n_out, 1u);
+    if (q >= A.ctl.out_cap) { atomicOr(A.ctl.err, VT_KERR_SUSPEND_FULL); return; }
+    const bool more = !SKIP || !(R.tent || R.ended);   /* a candidate to resume the walk at */
+    const unsigned int depth = more ? 1u : 0u, nsk = SKIP ? (unsigned int)R.nskip : 0u;
+    unsigned long long off = atomicAdd(A.ctl.pool_used, (unsigned long long)(depth + nsk));
+    SuspRec rec;
+    rec.ray = R.g;
+    if (off + depth + nsk <= A.ctl.pool_cap) {
+        for (unsigned int e = 0; e < nsk; e++) A.ctl.pool_out[off + e] = sk[e];
+        if (more) A.ctl.pool_out[off + nsk] = make_entry(0, A.oct.Lo, R.cx, R.cy, R.cz);
+        rec.depth = depth | (nsk << 8) | ((SKIP && R.tent ? 1u : 0u) << 11) | VT_SUSP_WALK |
+                    (R.taken << VT_SUSP_TAKEN_SHIFT);
+        rec.off = off;
+    } else {
+        /* pool full: as suspend_ray */
+        rec.depth = 0; rec.off = 0;
+    }
+    A.ctl.out[q] = rec;
+    if (SLAB && more && A.ctl.lookahead > 0) lookahead_walk(A, R, path);
+}
+
+/* A ray that left advance_trip: shades a hit (all lanes of a warp that have
+ * one together) and writes the pixel, suspends the ray, or hands it to the
+ * literal search. */
+template <int VTYPE, bool SLAB, int U, bool SKIP>
+__device__ __forceinline__ void finish_trip(const TraceArgs& A, const DevView* sv, Trip& R, uint2* path,
+                                            const unsigned long long* sk, int s, unsigned int* cnt) {
+    if (s == RAY_DONE || s == RAY_TENTATIVE || s == TRIP_MISS) {
+        Ray P;
+        P.rgba = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        P.hit = false; P.node = 0; P.brick = 0; P.t = -1.0f; P.n = f3(0, 0, 0);
+        P.view = R.view; P.i = R.i; P.j = R.j;
+        if (s != TRIP_MISS) {
+            const unsigned int x = R.cx, y = R.cy, z = R.cz, d = A.oct.Lo - A.oct.Lc;
+            Samp sm;
+            brick_sampler<VTYPE, SLAB>(A, x >> d, y >> d, z >> d, R.slot, sm);
+            P.r.o = R.r.o; P.dir = R.dir;
+            const float3 X = refine_hit<VTYPE, SLAB, false>(sm, R.dir, R.C, A.iso, A.refine, &cnt[VT_C_SAMPLES]);
+            shade_hit<VTYPE, SLAB, false>(A, P, sm, X, x, y, z, x >> d, y >> d, z >> d, cnt);
+        }
+        write_ray(A, sv, P, cnt, s != RAY_TENTATIVE);
+    }
+    if (s == RAY_TENTATIVE) R.tent = true;
+    if (s == RAY_SUSPENDED || (SKIP && s == RAY_TENTATIVE)) suspend_trip<SLAB, SKIP>(A, R, path, sk, cnt);
+    else if (SKIP && s == RAY_DONE_WRITTEN) cnt[VT_C_HITS]++;   /* the tentative hit stands */
+}
+
+/* record of a ray for the literal search: as it came in (a saved stack), or
+ * from the root past the candidates taken */
+__device__ __forceinline__ SuspRec literal_rec(const SuspRec& in, const Trip& R) {
+    SuspRec rec = in;
+    if (!in.depth || (in.depth & VT_SUSP_WALK)) rec.depth = VT_SUSP_WALK | (R.taken << VT_SUSP_TAKEN_SHIFT);
+    return rec;
+}
+
+/* adds a warp's counters to the CTA's */
+__device__ __forceinline__ void warp_counters(unsigned int* s_cnt, const unsigned int* cnt) {
+#pragma unroll
+    for (int c = 0; c < VT_C_COUNT; c++) {
+        const unsigned int v = c == VT_C_MAXSTACK ? __reduce_max_sync(0xffffffffu, cnt[c]) : __reduce_add_sync(0xffffffffu, cnt[c]);
+        if ((threadIdx.x & 31) == 0 && v) {
+            if (c == VT_C_MAXSTACK) atomicMax(&s_cnt[c], v);
+            else atomicAdd(&s_cnt[c], v);
+        }
+    }
+}
+
+/* One ray per lane, `group` rays a warp (a tile of the screen); a warp's rays
+ * walk, march and, at the end, shade together.  Bound by instruction issue
+ * and divergence (1920x1080 frame of the 512^3 blobs, warm: 67 % issue
+ * active, 15 of 32 lanes per instruction, 356 M warp instructions) and, on
+ * small frames, by the latency of the slowest warp.  Seven CTAs of 128
+ * threads per SM (72 registers): 5 CTAs 651 us, 6 627, 7 617, 8 634, 10 699
+ * on that frame.  Against the binary depth-first search it replaces: 767 ->
+ * 608 us there, 4.18 -> 3.55 ms for 16 mixed views, 769 -> 446 us for a
+ * 1277x719 uint8 frame with bisection, 94 -> 49 us for a 96x96 frame. */
+template <int VTYPE, bool SLAB, int U, bool SKIP>
+__global__ void __launch_bounds__(VT_TRACE_THREADS, VT_TRACE_CTAS) k_trace(const __grid_constant__ TraceArgs A) {
+    __shared__ uint2 s_path[VT_TREE64_LEVELS * VT_TRACE_THREADS];   /* per thread: the node entered at each level */
+    __shared__ unsigned int s_cnt[VT_C_COUNT];
+    uint2* const path = s_path + threadIdx.x;
+    if (threadIdx.x < VT_C_COUNT) s_cnt[threadIdx.x] = 0;
     __syncthreads();
+    const DevView* const sv = A.views.v;
+    const unsigned int nItems =
+        A.ctl.in ? (A.ctl.n_in_dev ? min(*A.ctl.n_in_dev, A.ctl.n_in) : A.ctl.n_in) : A.views.totalRays;
+    const unsigned int lane = threadIdx.x & 31;
+    const unsigned int w = (unsigned int)(blockIdx.x * (VT_TRACE_THREADS / 32) + (threadIdx.x >> 5)) * A.group + lane;
     unsigned int cnt[VT_C_COUNT];
 #pragma unroll
     for (int c = 0; c < VT_C_COUNT; c++) cnt[c] = 0;
-    const unsigned int nItems =
-        A.ctl.in ? (A.ctl.n_in_dev ? min(*A.ctl.n_in_dev, A.ctl.n_in) : A.ctl.n_in) : A.views.totalRays;
-    Stk st;
-    Ray R;
-    if (!PERSIST) {
-        unsigned int w = blockIdx.x * blockDim.x + threadIdx.x;
-        if (w < nItems) {
-            int s = start_ray<VTYPE, SKIP>(A, sv, w, R, st, cnt);
-            if (s == RAY_RUNNING) s = run_ray<VTYPE, SLAB, U, SKIP>(A, R, st, cnt, -1);
-            if (s == RAY_DONE) write_ray(A, sv, R, cnt);
-            else if (SKIP && s == RAY_TENTATIVE) {
-                write_ray(A, sv, R, cnt, false);
-                suspend_ray<VTYPE, SLAB, SKIP>(A, R, st, cnt);
-            } else if (s == RAY_SUSPENDED) suspend_ray<VTYPE, SLAB, SKIP>(A, R, st, cnt);
-            else if (SKIP && s == RAY_DONE_WRITTEN) cnt[VT_C_HITS]++;   /* the tentative hit stands */
-        }
-    } else {
-        const unsigned int lane = threadIdx.x & 31;
-        bool has = false;
-        for (;;) {
-            unsigned int need = __ballot_sync(0xffffffffu, !has);
-            if (need) {
-                unsigned int base = 0;
-                int leader = __ffs(need) - 1;
-                if ((int)lane == leader) base = atomicAdd(A.ctl.work, (unsigned int)__popc(need));
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (base >= nItems && need == 0xffffffffu) break;   /* queue drained, warp idle */
-                if (!has) {
-                    unsigned int w = base + __popc(need & ((1u << lane) - 1u));
-                    if (w < nItems) {
-                        int s = start_ray<VTYPE, SKIP>(A, sv, w, R, st, cnt);
-                        has = s == RAY_RUNNING;
-                        if (s == RAY_DONE) write_ray(A, sv, R, cnt);
-                    }
-                }
-            }
-            if (has) {
-                int s = run_ray<VTYPE, SLAB, U, SKIP>(A, R, st, cnt, A.pops);
-                if (s == RAY_DONE) { write_ray(A, sv, R, cnt); has = false; }
-                else if (SKIP && s == RAY_TENTATIVE) {
-                    write_ray(A, sv, R, cnt, false);
-                    suspend_ray<VTYPE, SLAB, SKIP>(A, R, st, cnt);
-                    has = false;
-                } else if (s == RAY_SUSPENDED) { suspend_ray<VTYPE, SLAB, SKIP>(A, R, st, cnt); has = false; }
-                else if (SKIP && s == RAY_DONE_WRITTEN) { cnt[VT_C_HITS]++; has = false; }   /* the tentative hit stands */
-            }
-        }
+    unsigned long long sk[VT_SKIP_MAX];
+    Trip R;
+    SuspRec rec;
+    int s = -1;
+    if (lane < A.group && w < nItems) {
+        if (A.ctl.in) rec = A.ctl.in[w];
+        else { rec.ray = w; rec.depth = 0; }
+        s = start_trip<SKIP>(A, sv, rec, R, path, sk);
+        if (s >= 0 && !A.ctl.in) cnt[VT_C_RAYS]++;
+        if (s == RAY_RUNNING) s = advance_trip<VTYPE, SLAB, U, SKIP>(A, R, path, sk, cnt);
     }
-    flush_counters(A, cnt);
+    __syncwarp();
+    if (s >= 0) finish_trip<VTYPE, SLAB, U, SKIP>(A, sv, R, path, sk, s, cnt);
+    if (s == TRIP_LITERAL) literal_ray<VTYPE, SLAB, U, SKIP>(A, sv, literal_rec(rec, R), R.nskip, sk);
+    __syncwarp();
+    warp_counters(s_cnt, cnt);
+    __syncthreads();
+    if (threadIdx.x < VT_C_COUNT) {
+        const int c = threadIdx.x;
+        unsigned int v = s_cnt[c];
+        if (SLAB && c == VT_C_DEVHITS) v = s_cnt[VT_C_CANDIDATES];
+        if (c == VT_C_MAXSTACK) v = s_cnt[VT_C_CANDIDATES] ? (unsigned int)(A.oct.Lo + 1) >> 1 : 0u;
+        if (v && c == VT_C_MAXSTACK) atomicMax(&A.ctl.counters[c], (unsigned long long)v);
+        else if (v) atomicAdd(&A.ctl.counters[c], (unsigned long long)v);
+    }
 }
 
 /* ---- wavefront passes ------------------------------------------------- */
@@ -759,8 +1009,12 @@ __global__ void __launch_bounds__(128, 8) k_wf_traverse(TraceArgs A, WaveRound W
     Stk st;
     Ray R;
     for (unsigned int w = blockIdx.x * blockDim.x + threadIdx.x; w < nItems; w += gridDim.x * blockDim.x) {
-        const int s0 = start_ray<VTYPE, false>(A, sv, w, R, st, cnt);
+        SuspRec rec0;
+        if (A.ctl.in) rec0 = A.ctl.in[w];
+        else { rec0.ray = w; rec0.depth = 0; }
+        const int s0 = start_ray<false>(A, sv, rec0, R, st);
         if (s0 < 0) continue;
+        if (!A.ctl.in) cnt[VT_C_RAYS]++;
         if (s0 == RAY_DONE) { write_ray(A, sv, R, cnt); continue; }
         for (;;) {
             bool stop = false;
@@ -773,6 +1027,7 @@ __global__ void __launch_bounds__(128, 8) k_wf_traverse(TraceArgs A, WaveRound W
                 if (!expand(A, R.r, st, R.top, e, cnt, true)) { stop = true; break; }
             }
             if (stop) { write_ray(A, sv, R, cnt); break; }   /* exhausted (or stack overflow, flagged) */
+            if (R.taken) { R.taken--; R.top--; continue; }
             const unsigned long long ent = st.e[R.top];
             const unsigned int x = e_x(ent), y = e_y(ent), z = e_z(ent);
             const unsigned int bx = x >> (Lo - Lc), by = y >> (Lo - Lc), bz = z >> (Lo - Lc);
@@ -811,13 +1066,11 @@ __global__ void __launch_bounds__(128, 8) k_wf_traverse(TraceArgs A, WaveRound W
             }
             /* no room to wait: march here */
             Samp sm;
-            int sl;
-            setup_sampler<VTYPE, true>(A, bx, by, bz, pidx, sm, &sl);
-            float3 X;
-            unsigned int ns = 0;
-            const bool h = march<VTYPE, true, 1>(sm, R.r.o, R.dir, tn, max_steps(tn, tf), A.iso, A.refine, &X, &ns);
-            cnt[VT_C_SAMPLES] += ns;
-            if (h) {
+            brick_sampler<VTYPE, true>(A, bx, by, bz, slot, sm);
+            Crossing C;
+            if (march<VTYPE, true, 1>(sm, R.r.o, R.dir, tn, max_steps(tn, tf), A.iso, C,
+                                      &cnt[VT_C_SAMPLES])) {
+                const float3 X = refine_hit<VTYPE, true, false>(sm, R.dir, C, A.iso, A.refine, &cnt[VT_C_SAMPLES]);
                 shade_hit<VTYPE, true, false>(A, R, sm, X, x, y, z, bx, by, bz, cnt);
                 write_ray(A, sv, R, cnt);
                 break;
@@ -931,11 +1184,9 @@ __global__ void __launch_bounds__(128) k_wf_march(TraceArgs A, WaveRound W, unsi
             sm.ox = (float)((int)(bx << sh) - B.inc); sm.oy = (float)((int)(by << sh) - B.inc);
             sm.oz = (float)((int)(bz << sh) - B.inc);
             sm.h = (float)(B.D - 2);
-            float3 X;
-            unsigned int ns = 0;
-            const bool h = march<VTYPE, true, 1, true>(sm, R.r.o, R.dir, it.tn, it.maxStep, A.iso, A.refine, &X, &ns);
-            cnt[VT_C_SAMPLES] += ns;
-            if (h) {
+            Crossing C;
+            if (march<VTYPE, true, 1, true>(sm, R.r.o, R.dir, it.tn, it.maxStep, A.iso, C, &cnt[VT_C_SAMPLES])) {
+                const float3 X = refine_hit<VTYPE, true, true>(sm, R.dir, C, A.iso, A.refine, &cnt[VT_C_SAMPLES]);
                 shade_hit<VTYPE, true, true>(A, R, sm, X, x, y, z, bx, by, bz, cnt);
                 write_ray(A, sv, R, cnt);
             } else {
@@ -1096,41 +1347,37 @@ cudaError_t vt_launch_predict_requests(int* page, const unsigned int* leafPages,
     return cudaGetLastError();
 }
 
-cudaError_t vt_launch_trace(const TraceArgs& a, bool slabMode, bool persistent, int blocksPerSM, cudaStream_t s) {
-    const int threads = 128;
-    unsigned int items = a.ctl.in ? a.ctl.n_in : a.views.totalRays;
+cudaError_t vt_launch_trace(const TraceArgs& a0, bool slabMode, cudaStream_t s) {
+    const unsigned int items = a0.ctl.in ? a0.ctl.n_in : a0.views.totalRays;
     if (items == 0) return cudaSuccess;
-    if (a.views.n < 1 || a.views.n > VT_MAX_VIEWS) return cudaErrorInvalidValue;
-    unsigned int blocks;
-    if (persistent) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        unsigned int want = (items + threads - 1) / threads;
-        blocks = (unsigned int)(sms * (blocksPerSM > 0 ? blocksPerSM : 8));
-        if (blocks > want) blocks = want;
-    } else {
-        blocks = (items + threads - 1) / threads;
-    }
+    if (a0.views.n < 1 || a0.views.n > VT_MAX_VIEWS) return cudaErrorInvalidValue;
+    TraceArgs a = a0;
+    /* a full warp a tile, unless that leaves the GPU short of warps: then
+     * fewer rays a warp, which diverge less.  A warp's time is the sum of its
+     * lanes' separate turns, so on a 96x96 frame (288 full warps for 4144
+     * places) 32, 16, 8, 4, 1 rays a warp took 74, 61, 50, 49, 45 us. */
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const unsigned int places = (unsigned int)sms * VT_TRACE_CTAS * (VT_TRACE_THREADS / 32);
+    a.group = 32;
+    while (a.group > 1 && items / a.group < places) a.group >>= 1;
+    const unsigned long long warps = (items + (unsigned long long)a.group - 1) / a.group;
+    const unsigned int blocks = (unsigned int)((warps + VT_TRACE_THREADS / 32 - 1) / (VT_TRACE_THREADS / 32));
     /* setting absent bricks aside is compiled into its own kernels, so the
      * in-order traversal keeps its registers; it needs bricks (slab mode)
      * and is off while a trace is logged */
     const bool skip = slabMode && a.ctl.skip > 0 && !a.ctl.touched;
-#define VT_LAUNCH_U(V, S, P, K)                                            \
-    switch (a.unroll) {                                                    \
-        case 2: k_trace<V, S, P, 2, K><<<blocks, threads, 0, s>>>(a); break; \
-        case 4: k_trace<V, S, P, 4, K><<<blocks, threads, 0, s>>>(a); break; \
-        case 8: k_trace<V, S, P, 8, K><<<blocks, threads, 0, s>>>(a); break; \
-        default: k_trace<V, S, P, 1, K><<<blocks, threads, 0, s>>>(a); break; \
+#define VT_LAUNCH_U(V, S, K)                                                     \
+    switch (a.unroll) {                                                          \
+        case 2: k_trace<V, S, 2, K><<<blocks, VT_TRACE_THREADS, 0, s>>>(a); break; \
+        case 4: k_trace<V, S, 4, K><<<blocks, VT_TRACE_THREADS, 0, s>>>(a); break; \
+        case 8: k_trace<V, S, 8, K><<<blocks, VT_TRACE_THREADS, 0, s>>>(a); break; \
+        default: k_trace<V, S, 1, K><<<blocks, VT_TRACE_THREADS, 0, s>>>(a); break; \
     }
-#define VT_LAUNCH(V, S, P) { if (S && skip) VT_LAUNCH_U(V, S, P, S) else VT_LAUNCH_U(V, S, P, false) }
-    if (a.br.vtype == 0) {
-        if (slabMode) { if (persistent) VT_LAUNCH(0, true, true) else VT_LAUNCH(0, true, false) }
-        else { if (persistent) VT_LAUNCH(0, false, true) else VT_LAUNCH(0, false, false) }
-    } else {
-        if (slabMode) { if (persistent) VT_LAUNCH(1, true, true) else VT_LAUNCH(1, true, false) }
-        else { if (persistent) VT_LAUNCH(1, false, true) else VT_LAUNCH(1, false, false) }
-    }
+#define VT_LAUNCH(V, S) { if (S && skip) VT_LAUNCH_U(V, S, S) else VT_LAUNCH_U(V, S, false) }
+    if (a.br.vtype == 0) { if (slabMode) VT_LAUNCH(0, true) else VT_LAUNCH(0, false) }
+    else { if (slabMode) VT_LAUNCH(1, true) else VT_LAUNCH(1, false) }
 #undef VT_LAUNCH_U
 #undef VT_LAUNCH
     return cudaGetLastError();

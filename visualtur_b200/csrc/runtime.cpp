@@ -21,6 +21,7 @@
 #include "vt_kernels.h"
 #include "vt_runtime.h"
 #include "cache.h"
+#include "tree64_build.h"
 #include "vt_math.cuh"
 
 using namespace vtrt;
@@ -147,7 +148,7 @@ extern "C" vt_status vt_render_cube(const vt_camera* c, const float* dev_cube, c
 struct CtlBlock {
     unsigned long long counters[VT_C_COUNT];
     unsigned int err;
-    unsigned int n_out, n_req, work;       /* reset every pass */
+    unsigned int n_out, n_req;             /* reset every pass */
     unsigned long long pool_used;
 };
 
@@ -161,6 +162,7 @@ struct vt_handle {
     int nLevels = 0, Lo = 0, Lc = 0, inc = 3, edge = 0, D = 0;
     /* flattened octree */
     uint2* d_nodes = nullptr;
+    uint4* d_nodes64 = nullptr;         /* the same tree two levels at a time */
     size_t nodeCount = 0;
     int rootValid = 0;
     std::vector<uint64_t> leafBricks;   /* bricks holding reachable candidate nodes */
@@ -283,6 +285,9 @@ static vt_status flatten_octree(vt_handle* h) {
     h->nodeCount = all.size();
     CK(cudaMalloc(&h->d_nodes, std::max<size_t>(all.size(), 1) * sizeof(uint2)));
     CK(cudaMemcpy(h->d_nodes, all.data(), all.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+    const std::vector<uint4> t64 = vt::build_tree64(all, Lo);
+    CK(cudaMalloc(&h->d_nodes64, t64.size() * sizeof(uint4)));
+    CK(cudaMemcpy(h->d_nodes64, t64.data(), t64.size() * sizeof(uint4), cudaMemcpyHostToDevice));
     /* bricks that hold reachable candidates, as Morton codes at levelCubes */
     const int shift = 3 * (Lo - h->Lc);
     h->leafBricks.clear();
@@ -474,7 +479,7 @@ extern "C" void vt_destroy(vt_handle* h) {
     if (h->s_int) cudaStreamSynchronize(h->s_int);
     cudaDeviceSynchronize();
     free_ray_buffers(h);
-    cudaFree(h->d_nodes);
+    cudaFree(h->d_nodes); cudaFree(h->d_nodes64);
     for (int i = 0; i < 2; i++) { cudaFree(h->d_susp[i]); cudaFree(h->d_pool[i]); }
     cudaFree(h->d_vol); cudaFree(h->d_ctl); cudaFree(h->d_views); cudaFree(h->d_req); cudaFree(h->d_touched);
     if (h->h_ctl) cudaFreeHost(h->h_ctl);
@@ -558,6 +563,7 @@ static void fill_args(vt_handle* h, TraceArgs& a, int nViews, unsigned int total
     a.views.v = h->d_views; a.views.n = nViews; a.views.totalRays = totalRays;
     a.oct.nLevels = h->nLevels; a.oct.Lo = h->Lo; a.oct.Lc = h->Lc; a.oct.rootValid = h->rootValid;
     a.oct.nodes = h->d_nodes;
+    a.oct.t64.nodes = h->d_nodes64; a.oct.t64.nLevels = h->nLevels; a.oct.t64.Lo = h->Lo;
     a.br.vtype = h->vol->vtype; a.br.inc = h->inc;
     if (h->opt.resident) {
         a.br.vol = h->d_vol; a.br.P = h->P; a.br.ve = (int)h->ve;
@@ -567,7 +573,7 @@ static void fill_args(vt_handle* h, TraceArgs& a, int nViews, unsigned int total
     }
     if (nViews == 1) { a.out.node = h->d_node; a.out.brick = h->d_brick; a.out.t = h->d_t; a.out.n = h->d_n; }
     CtlBlock* c = h->d_ctl;
-    a.ctl.counters = c->counters; a.ctl.err = &c->err; a.ctl.work = &c->work;
+    a.ctl.counters = c->counters; a.ctl.err = &c->err;
     a.ctl.n_out = &c->n_out; a.ctl.n_req = &c->n_req; a.ctl.pool_used = &c->pool_used;
     a.ctl.req = h->d_req; a.ctl.req_cap = h->req_cap;
     a.ctl.lookahead = h->opt.lookahead;
@@ -580,7 +586,6 @@ static void fill_args(vt_handle* h, TraceArgs& a, int nViews, unsigned int total
     a.iso = h->oct->iso;
     a.light = make_float3(0.0f, 512.0f, 0.0f);   /* src/visualTur.cu:30 */
     a.tile_w = h->opt.tile_w; a.tile_h = h->opt.tile_h;
-    a.pops = h->opt.pops > 0 ? h->opt.pops : 8;
     a.unroll = h->opt.unroll;
     a.refine = h->opt.refine;
 }
@@ -648,12 +653,12 @@ static vt_status ensure_wave_buffers(vt_handle* h, unsigned int rays) {
 }
 
 /* One pass's kernels: the fused trace kernel, or wavefront rounds then the
- * fused kernel (persistent, its ray count read on the device) for the rays
+ * fused kernel (its ray count read on the device) for the rays
  * still waiting.  `bound`: rays the pass can hold (wavefront buffers). */
 static cudaError_t launch_pass(vt_handle* h, const TraceArgs& a0, bool slabMode, cudaStream_t s, int* kernels) {
     if (!use_wave(h, slabMode)) {
         *kernels = 1;
-        return vt_launch_trace(a0, slabMode, h->opt.persistent != 0, h->opt.blocks_per_sm, s);
+        return vt_launch_trace(a0, slabMode, s);
     }
     const int rounds = h->opt.wavefront;
     const unsigned int bound = h->wave_cap;
@@ -682,7 +687,7 @@ static cudaError_t launch_pass(vt_handle* h, const TraceArgs& a0, bool slabMode,
     const int p = (rounds - 1) & 1;
     a.ctl.in = h->d_wnext[p]; a.ctl.n_in = bound; a.ctl.pool_in = h->d_wpool[p]; a.ctl.n_in_dev = &h->d_wctl[p].n_next;
     *kernels = 4 * rounds + 1;
-    return vt_launch_trace(a, slabMode, true, h->opt.blocks_per_sm, s);
+    return vt_launch_trace(a, slabMode, s);
 }
 
 /* pass 0: clear the control block (and trace log), upload the view table,

@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tree64.cuh"
+
 #define VT_MAX_LEVELS 20
 #define VT_STACK 64          /* per-ray DFS stack entries (reference: 32) */
 #define VT_SKIP_MAX 4        /* absent-brick candidates a ray may pass over in one pass */
@@ -36,10 +38,14 @@ struct DevCamera {
 /* Flattened octree: records of the reachable nodes of levels 0..Lo-1 in
  * one array, level after level.  node.x = array index of the first child,
  * node.y = 8-bit child mask (bit k = child (code<<3)+k accepted by the
- * reference's range search); children of a node are contiguous. */
+ * reference's range search); children of a node are contiguous.  t64 holds
+ * the same nodes two levels at a time (tree64.cuh), which the trace kernel
+ * walks; the binary nodes serve rays the walk hands back (WALK_TIE) and the
+ * wavefront passes. */
 struct DevOctree {
     int nLevels, Lo, Lc, rootValid;
     const uint2* nodes;
+    vt::Tree64 t64;
 };
 
 /* DFS stack entry (8 bytes): node array index, level, and the node's
@@ -90,7 +96,11 @@ struct DevViews {
  * from the root) and offset of its entries in the stack pool. */
 /* A suspended ray: its pool entries at `off` are its passed-over
  * candidates (depth bits 8-10), then its DFS stack (bits 0-7); bit 11: its
- * pixel already holds a hit found past those candidates. */
+ * pixel already holds a hit found past those candidates; bit 12: instead of
+ * a stack the entry is the candidate the 64-ary walk stopped at, and bits
+ * 13-31 count the candidates taken before it (at most 3 * 2^octreeLevel). */
+#define VT_SUSP_WALK (1u << 12)
+#define VT_SUSP_TAKEN_SHIFT 13
 struct SuspRec {
     unsigned int ray;
     unsigned int depth;
@@ -101,7 +111,6 @@ struct SuspRec {
 struct DevCtl {
     unsigned long long* counters;
     unsigned int* err;
-    unsigned int* work;                         /* persistent-kernel work counter */
     const SuspRec* in; unsigned int n_in;      /* rays to resume (NULL: pass 0) */
     const unsigned int* n_in_dev;               /* if set: the count, in device memory (n_in bounds it) */
     const unsigned long long* pool_in;
@@ -123,7 +132,7 @@ struct TraceArgs {
     float iso;
     float3 light;
     int tile_w, tile_h;
-    int pops;                                   /* pops between warp refills (persistent) */
+    unsigned int group;                         /* rays a warp takes (32 or, where they are few, less) */
     int unroll;                                 /* march samples fetched per round: 1, 2, 4, 8 */
     int refine;                                 /* bisection steps before the linear refinement */
 };
@@ -162,7 +171,7 @@ struct WaveRound {
 };
 
 /* launchers (render.cu) */
-cudaError_t vt_launch_trace(const TraceArgs& a, bool slab, bool persistent, int blocks_per_sm, cudaStream_t s);
+cudaError_t vt_launch_trace(const TraceArgs& a, bool slab, cudaStream_t s);
 cudaError_t vt_launch_wave_round(const TraceArgs& a, const WaveRound& w, int blocks_per_sm, size_t slotBytes,
                                  cudaStream_t s);
 cudaError_t vt_launch_rays(const DevCamera& c, float* dirs, cudaStream_t s);
