@@ -14,18 +14,20 @@
  *   root     = {1,1} when level 1 has children of node 1 (:532-540);
  *   a level  = its valid codes as sorted inclusive runs [s,e] (insert /
  *              completeLevel, :79-128).
- * The GPU version keeps each level as a bitmask over its Morton codes, turns
- * runs of ones into [s,e] pairs with two prefix sums, and runs the builder's
- * search only for parents that have a set child byte (the search never
- * finds a child a range does not hold).  Output is byte-identical to the
- * reference's volumeToOctree.
+ * The GPU version keeps each level as a bitmask over its Morton codes and
+ * counts run starts with a prefix sum; a parent's range search follows from
+ * the count before its children and their bits alone (vt_search.h,
+ * has_children_rank), so no level waits for the ranges of the one below and
+ * the host is asked for nothing until all levels are done.  The ranges are
+ * then made, copied back and written window by window.
+ * Output is byte-identical to the reference's volumeToOctree.
  */
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
 
-#include <cub/cub.cuh>
-#include <vector>
+#include <algorithm>
+#include <memory>
 
 #include "../../include/vt.h"
 #include "vt_math.cuh"
@@ -40,172 +42,217 @@ namespace vtb {
         if (e_ != cudaSuccess) { st = vtrt::fail(VT_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); goto done; } \
     } while (0)
 
+/* Leaf cells of one 8 x 8 x 64 box (x, y, z) per CTA turn (src/CreateOctree.cu:471-517):
+ * bit b of word w = cell with Morton offset 32w + b.  Each voxel row of the
+ * box and its far faces (9 x 9 rows of 65) becomes sign bits by ballots, a
+ * row of cells is then an AND and an OR of four rows and their shifts (all
+ * eight corners alike or not), and 128 threads gather the words, 2 x 4 x 4
+ * cells each.  Bound by memory: a voxel is read 1.3 times, by whole 128-byte
+ * lines.  Against one thread per word reading eight corners per cell: 512^3
+ * float32 1003 -> 283 us, 201 x 333 x 129 uint8 (in its 512^3 cube)
+ * 994 -> 33 us. */
+#define LB_X 8
+#define LB_Y 8
+#define LB_Z 64
 template <int VTYPE>
-__device__ __forceinline__ float vox(const void* v, long long dx, long long dy, long long dz, long long x, long long y,
-                                     long long z) {
-    if (x >= dx || y >= dy || z >= dz) return 0.0f;   /* zero padding (x,y,z >= 0 here) */
-    long long i = (x * dy + y) * dz + z;
-    if (VTYPE == 0) return __ldg((const float*)v + i);
-    return (float)__ldg((const unsigned char*)v + i);
+__global__ void __launch_bounds__(256) k_leaf(const void* v, long long dx, long long dy, long long dz, float iso,
+                                              uint32_t* bits, int N, long long nby, long long nbz, long long boxes) {
+    __shared__ unsigned long long row[LB_X + 1][LB_Y + 1];
+    __shared__ unsigned char ext[LB_X + 1][LB_Y + 1];          /* the sign behind the row's end */
+    __shared__ unsigned long long cells[LB_X][LB_Y];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool zero = (0.0f - iso) < 0;                        /* zero padding */
+    for (long long box = blockIdx.x; box < boxes; box += gridDim.x) {
+        const long long z0 = box % nbz * LB_Z, y0 = box / nbz % nby * LB_Y, x0 = box / nbz / nby * LB_X;
+        for (int r = warp; r < (LB_X + 1) * (LB_Y + 1); r += 8) {
+            const int rx = r / (LB_Y + 1), ry = r % (LB_Y + 1);
+            const long long x = x0 + rx, y = y0 + ry;
+            bool s0 = zero, s1 = zero, s2 = zero;
+            if (x < dx && y < dy) {
+                const long long i = (x * dy + y) * dz + z0;
+                const long long left = dz - z0;                /* voxels of the row from z0 on */
+                if (VTYPE == 0) {
+                    const float* p = (const float*)v + i;
+                    float a = 0.0f, b = 0.0f, c = 0.0f;
+                    if (lane < left) a = __ldg(p + lane);
+                    if (lane + 32 < left) b = __ldg(p + lane + 32);
+                    if (lane == 0 && left > LB_Z) c = __ldg(p + LB_Z);
+                    s0 = (a - iso) < 0; s1 = (b - iso) < 0; s2 = (c - iso) < 0;
+                } else {
+                    const unsigned char* p = (const unsigned char*)v + i;
+                    unsigned int a = 0, b = 0, c = 0;
+                    if (lane < left) a = __ldg(p + lane);
+                    if (lane + 32 < left) b = __ldg(p + lane + 32);
+                    if (lane == 0 && left > LB_Z) c = __ldg(p + LB_Z);
+                    s0 = ((float)a - iso) < 0; s1 = ((float)b - iso) < 0; s2 = ((float)c - iso) < 0;
+                }
+            }
+            const unsigned int lo = __ballot_sync(0xffffffffu, s0), hi = __ballot_sync(0xffffffffu, s1);
+            if (lane == 0) { row[rx][ry] = (unsigned long long)hi << 32 | lo; ext[rx][ry] = s2; }
+        }
+        __syncthreads();
+        if (tid < LB_X * LB_Y) {
+            const int cx = tid / LB_Y, cy = tid % LB_Y;
+            unsigned long long all = ~0ull, any = 0;
+            unsigned long long allE = 1, anyE = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const unsigned long long m = row[cx + (k >> 1)][cy + (k & 1)], e = ext[cx + (k >> 1)][cy + (k & 1)];
+                all &= m; any |= m; allE &= e; anyE |= e;
+            }
+            cells[cx][cy] = (any | (any >> 1 | anyE << 63)) & ~(all & (all >> 1 | allE << 63));
+        }
+        __syncthreads();
+        if (tid < (LB_X / 2) * (LB_Y / 4) * (LB_Z / 4)) {
+            /* 16 consecutive words make an 8^3 block: x1, z2, y2, x2 of the cell from the low bit up */
+            const int X = ((tid & 1) << 1) | ((tid & 8) >> 1), Z = ((tid & 2) << 1) | ((tid >> 4) << 3), Y = tid & 4;
+            if (x0 + X < N && y0 + Y < N && z0 + Z < N) {
+                uint32_t m = 0;
+#pragma unroll
+                for (int x = 0; x < 2; x++)
+#pragma unroll
+                    for (int y = 0; y < 4; y++) {
+                        const uint32_t q = (uint32_t)(cells[X + x][Y + y] >> Z) & 15u;   /* four cells in z */
+                        m |= ((q & 3u) | (q & 12u) << 6) << (4 * x + 2 * (y & 1) + 16 * (y >> 1));
+                    }
+                const uint64_t off = (vt::spread3((uint32_t)(x0 + X)) << 2) | (vt::spread3((uint32_t)(y0 + Y)) << 1) |
+                                     vt::spread3((uint32_t)(z0 + Z));
+                bits[off >> 5] = m;
+            }
+        }
+        __syncthreads();
+    }
 }
 
-/* leaf cells: bit b of word w = cell with Morton offset 32w+b (src/CreateOctree.cu:471-517) */
-template <int VTYPE>
-__global__ void k_leaf(const void* v, long long dx, long long dy, long long dz, float iso, uint32_t* bits,
-                       long long nwords) {
-    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < nwords;
-         w += (long long)gridDim.x * blockDim.x) {
-        uint32_t m = 0;
-        for (int b = 0; b < 32; b++) {
-            uint64_t off = (uint64_t)w * 32 + b;
-            long long x = vt::compact3(off >> 2), y = vt::compact3(off >> 1), z = vt::compact3(off);
-            float c[8];
-            c[0] = vox<VTYPE>(v, dx, dy, dz, x, y, z);         c[1] = vox<VTYPE>(v, dx, dy, dz, x, y, z + 1);
-            c[2] = vox<VTYPE>(v, dx, dy, dz, x, y + 1, z);     c[3] = vox<VTYPE>(v, dx, dy, dz, x, y + 1, z + 1);
-            c[4] = vox<VTYPE>(v, dx, dy, dz, x + 1, y, z);     c[5] = vox<VTYPE>(v, dx, dy, dz, x + 1, y, z + 1);
-            c[6] = vox<VTYPE>(v, dx, dy, dz, x + 1, y + 1, z); c[7] = vox<VTYPE>(v, dx, dy, dz, x + 1, y + 1, z + 1);
-            bool sign = (c[0] - iso) < 0;
-            bool has = false;
-            for (int i = 1; i < 8; i++) has |= (((c[i] - iso) < 0) != sign);
-            m |= (uint32_t)has << b;
-        }
-        bits[w] = m;
-    }
+/* one level on the device */
+struct Level {
+    uint32_t* bits;                 /* its codes as a bitmask (Morton offset i = bit i) */
+    uint32_t* offs;                 /* per word: run starts before it in its block of CB_WORDS words */
+    unsigned long long* block;      /* per block: run starts, then (k_scan) run starts before it */
+    unsigned long long* total;      /* run starts */
+    long long words, blocks;
+};
+#define CB_WORDS 2048
+
+/* runs that start before word w */
+__device__ __forceinline__ unsigned long long starts_before(const Level& L, long long w) {
+    return L.block[w / CB_WORDS] + L.offs[w];
+}
+/* the run starts / ends among word w's bits */
+__device__ __forceinline__ uint32_t run_starts(const Level& L, long long w, uint32_t m) {
+    return m & ~((m << 1) | (w > 0 ? L.bits[w - 1] >> 31 : 0u));
+}
+__device__ __forceinline__ uint32_t run_ends(const Level& L, long long w, uint32_t m) {
+    return m & ~((m >> 1) | (w + 1 < L.words ? L.bits[w + 1] << 31 : 0u));
 }
 
 /* inner level: parent p exists when it has a set child byte, is not the
- * level's last code, and the builder's search over level l+1 finds a child */
-__global__ void k_inner(const uint32_t* childBits, const uint64_t* e, long long n, uint64_t base, uint64_t lastOff,
-                        uint32_t* bits, long long nwords, long long nparents) {
-    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < nwords;
-         w += (long long)gridDim.x * blockDim.x) {
-        uint32_t m = 0;
-        for (int b = 0; b < 32; b++) {
-            long long p = w * 32 + b;
-            if (p >= nparents || (uint64_t)p == lastOff) continue;
-            uint32_t byte = (childBits[p >> 2] >> (8 * (p & 3))) & 0xFFu;
-            if (!byte) continue;
-            if (vtsearch::search_children_host(e, n, base + (uint64_t)p) > 0) m |= 1u << b;
+ * level's last code, and the builder's search over the child level finds a
+ * child.  One parent per lane, a word per warp. */
+__global__ void __launch_bounds__(256) k_inner(const Level C, uint32_t* bits, long long words, long long parents) {
+    const int64_t n = 2 * (int64_t)*C.total;
+    const int lane = threadIdx.x & 31;
+    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words;
+         w += ((long long)gridDim.x * blockDim.x) >> 5) {
+        const long long p = w * 32 + lane;
+        bool set = false;
+        if (p < parents - 1) {
+            const long long cw = p >> 2;
+            const uint32_t m = C.bits[cw];
+            const int sh = 8 * (int)(p & 3);
+            const uint32_t byte = (m >> sh) & 0xFFu;
+            if (byte) {
+                const uint32_t st = run_starts(C, cw, m);
+                set = vtsearch::has_children_rank(n, byte, (st >> sh) & 0xFFu,
+                                                  (int64_t)starts_before(C, cw) + __popc(st & ((1u << sh) - 1u)));
+            }
         }
-        bits[w] = m;
+        const uint32_t b = __ballot_sync(0xffffffffu, set);
+        if (lane == 0) bits[w] = b;
     }
 }
 
-/* run starts / ends per word (bit i of the level = Morton offset i) */
-__global__ void k_runcount(const uint32_t* bits, long long nwords, uint32_t* cs, uint32_t* ce) {
-    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < nwords;
-         w += (long long)gridDim.x * blockDim.x) {
-        uint32_t m = bits[w];
-        uint32_t prev = w > 0 ? bits[w - 1] >> 31 : 0u;
-        uint32_t next = w + 1 < nwords ? bits[w + 1] & 1u : 0u;
-        uint32_t starts = m & ~((m << 1) | prev);
-        uint32_t ends = m & ~((m >> 1) | (next << 31));
-        cs[w] = __popc(starts);
-        ce[w] = __popc(ends);
-    }
-}
-__global__ void k_runwrite(const uint32_t* bits, long long nwords, const unsigned long long* os,
-                           const unsigned long long* oe, uint64_t base, uint64_t* out) {
-    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < nwords;
-         w += (long long)gridDim.x * blockDim.x) {
-        uint32_t m = bits[w];
-        uint32_t prev = w > 0 ? bits[w - 1] >> 31 : 0u;
-        uint32_t next = w + 1 < nwords ? bits[w + 1] & 1u : 0u;
-        uint32_t starts = m & ~((m << 1) | prev);
-        uint32_t ends = m & ~((m >> 1) | (next << 31));
-        unsigned long long k = os[w];
-        while (starts) {
-            int b = __ffs(starts) - 1;
-            starts &= starts - 1;
-            out[2 * k++] = base + (uint64_t)w * 32 + b;
+/* run starts per word (exclusive within its block) and per block; eight
+ * words a thread */
+__global__ void __launch_bounds__(256) k_count(const Level L) {
+    __shared__ uint32_t warpSum[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (long long blk = blockIdx.x; blk < L.blocks; blk += gridDim.x) {
+        const long long w0 = blk * CB_WORDS + threadIdx.x * 8;
+        uint32_t c[8], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            c[k] = sum;
+            if (w0 + k < L.words) sum += __popc(run_starts(L, w0 + k, L.bits[w0 + k]));
         }
-        k = oe[w];
-        while (ends) {
-            int b = __ffs(ends) - 1;
-            ends &= ends - 1;
-            out[2 * k++ + 1] = base + (uint64_t)w * 32 + b;
+        uint32_t inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
         }
+        if (lane == 31) warpSum[warp] = inc;
+        __syncthreads();
+        uint32_t base = inc - sum, all = 0;
+        for (int k = 0; k < 8; k++) { if (k < warp) base += warpSum[k]; all += warpSum[k]; }
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (w0 + k < L.words) L.offs[w0 + k] = base + c[k];
+        if (threadIdx.x == 0) L.block[blk] = all;
+        __syncthreads();
     }
-}
-__global__ void k_widen(const uint32_t* a, unsigned long long* b, long long n) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        b[i] = a[i];
 }
 
-static unsigned int grid_for(long long n) {
-    long long g = (n + 255) / 256;
+/* block counts -> exclusive offsets, and the level's total (one CTA) */
+__global__ void __launch_bounds__(1024) k_scan(const Level L) {
+    __shared__ unsigned long long warpSum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long carry = 0;
+    for (long long b0 = 0; b0 < L.blocks; b0 += 1024) {
+        const long long b = b0 + threadIdx.x;
+        const unsigned long long v = b < L.blocks ? L.block[b] : 0ull;
+        unsigned long long inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        if (lane == 31) warpSum[warp] = inc;
+        __syncthreads();
+        unsigned long long before = carry, all = 0;
+        for (int k = 0; k < 32; k++) { if (k < warp) before += warpSum[k]; all += warpSum[k]; }
+        if (b < L.blocks) L.block[b] = before + inc - v;
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *L.total = carry;
+}
+
+/* words [k0, k1) of the level's inclusive ranges [s, e], in order: the run an
+ * end belongs to is the last one that starts at or before it */
+__global__ void __launch_bounds__(256) k_ranges(const Level L, uint64_t base, unsigned long long k0, unsigned long long k1,
+                                                uint64_t* out) {
+    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < L.words;
+         w += (long long)gridDim.x * blockDim.x) {
+        const uint32_t m = L.bits[w];
+        if (!m) continue;
+        const uint32_t starts = run_starts(L, w, m), ends = run_ends(L, w, m);
+        const unsigned long long before = starts_before(L, w);
+        unsigned long long k = 2 * before;
+        for (uint32_t s = starts; s; s &= s - 1, k += 2)
+            if (k >= k0 && k < k1) out[k - k0] = base + (uint64_t)w * 32 + (__ffs(s) - 1);
+        for (uint32_t e = ends; e; e &= e - 1) {
+            const int b = __ffs(e) - 1;
+            k = 2 * (before + __popc(starts & (0xFFFFFFFFu >> (31 - b)))) - 1;
+            if (k >= k0 && k < k1) out[k - k0] = base + (uint64_t)w * 32 + b;
+        }
+    }
+}
+#define RANGE_WINDOW (1ll << 19)   /* words made and copied at a time (4 MB) */
+
+static unsigned int grid_for(long long threads, int block) {
+    const long long g = (threads + block - 1) / block;
     return (unsigned int)(g < 148 * 32 ? (g < 1 ? 1 : g) : 148 * 32);
-}
-
-__global__ void k_addc(unsigned long long* a, long long n, unsigned long long c) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        a[i] += c;
-}
-
-/* exclusive prefix sums of two u32 count arrays into u64 offsets, in chunks
- * of 2^30 items (cub's item count is an int) with carried totals */
-static cudaError_t scan2(uint32_t* cs, uint32_t* ce, unsigned long long* os, unsigned long long* oe, long long n,
-                         cudaStream_t s, unsigned long long* ts, unsigned long long* te) {
-    cudaError_t e = cudaSuccess;
-    const long long CH = 1ll << 30;
-    k_widen<<<grid_for(n), 256, 0, s>>>(cs, os, n);
-    k_widen<<<grid_for(n), 256, 0, s>>>(ce, oe, n);
-    size_t tmp = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tmp, os, os, (int)(n < CH ? n : CH), s);
-    void* d_tmp = nullptr;
-    if ((e = cudaMalloc(&d_tmp, tmp + 16)) != cudaSuccess) return e;
-    unsigned long long carry[2] = {0, 0};
-    unsigned long long* h = nullptr;
-    if ((e = cudaMallocHost(&h, 4 * 8)) != cudaSuccess) { cudaFree(d_tmp); return e; }
-    for (long long o = 0; o < n && e == cudaSuccess; o += CH) {
-        int m = (int)(n - o < CH ? n - o : CH);
-        cudaMemcpyAsync(h + 0, os + o + m - 1, 8, cudaMemcpyDeviceToHost, s);   /* last counts */
-        cudaMemcpyAsync(h + 1, oe + o + m - 1, 8, cudaMemcpyDeviceToHost, s);
-        cub::DeviceScan::ExclusiveSum(d_tmp, tmp, os + o, os + o, m, s);
-        cub::DeviceScan::ExclusiveSum(d_tmp, tmp, oe + o, oe + o, m, s);
-        cudaMemcpyAsync(h + 2, os + o + m - 1, 8, cudaMemcpyDeviceToHost, s);   /* last offsets */
-        cudaMemcpyAsync(h + 3, oe + o + m - 1, 8, cudaMemcpyDeviceToHost, s);
-        if (carry[0]) k_addc<<<grid_for(m), 256, 0, s>>>(os + o, m, carry[0]);
-        if (carry[1]) k_addc<<<grid_for(m), 256, 0, s>>>(oe + o, m, carry[1]);
-        e = cudaStreamSynchronize(s);
-        carry[0] += h[2] + h[0];
-        carry[1] += h[3] + h[1];
-    }
-    cudaFree(d_tmp);
-    cudaFreeHost(h);
-    *ts = carry[0];
-    *te = carry[1];
-    if (e == cudaSuccess) e = cudaGetLastError();
-    return e;
-}
-
-/* bitmask -> device range array of the level; returns words (2 * runs) */
-static vt_status encode(const uint32_t* bits, long long nwords, uint64_t base, cudaStream_t s, uint64_t** out,
-                        long long* nout) {
-    vt_status st = VT_OK;
-    uint32_t *cs = nullptr, *ce = nullptr;
-    unsigned long long *os = nullptr, *oe = nullptr;
-    unsigned long long ts = 0, te = 0;
-    *out = nullptr;
-    *nout = 0;
-    CKB(cudaMalloc(&cs, nwords * 4));
-    CKB(cudaMalloc(&ce, nwords * 4));
-    CKB(cudaMalloc(&os, nwords * 8));
-    CKB(cudaMalloc(&oe, nwords * 8));
-    k_runcount<<<grid_for(nwords), 256, 0, s>>>(bits, nwords, cs, ce);
-    CKB(cudaGetLastError());
-    CKB(scan2(cs, ce, os, oe, nwords, s, &ts, &te));
-    if (ts != te) { st = vtrt::fail(VT_ERR_STATE, "run encoding mismatch (%llu starts, %llu ends)", ts, te); goto done; }
-    if (2 * ts > 0x7FFFFFFFull) { st = vtrt::fail(VT_ERR_UNSUPPORTED, "level with %llu ranges exceeds the file format", ts); goto done; }
-    if (ts) {
-        CKB(cudaMalloc(out, 2 * ts * 8));
-        k_runwrite<<<grid_for(nwords), 256, 0, s>>>(bits, nwords, os, oe, base, *out);
-        CKB(cudaGetLastError());
-    }
-    *nout = (long long)(2 * ts);
-done:
-    cudaFree(cs); cudaFree(ce); cudaFree(os); cudaFree(oe);
-    return st;
 }
 
 }  // namespace vtb
@@ -229,61 +276,102 @@ extern "C" vt_status vt_octree_build_device(const void* dev_vol, int vtype, cons
     int nLevels = aux2 > 0.0 ? (int)(aux + 1) : (int)aux;
     dimension = (int)pow(2, nLevels);
     if (nLevels < 1 || nLevels > 13) return vtrt::fail(VT_ERR_UNSUPPORTED, "volume extent gives %d levels", nLevels);
-    std::vector<std::vector<uint64_t> > levels(nLevels + 1);
-    uint32_t* childBits = nullptr;
-    uint64_t* childRanges = nullptr;
-    long long childN = 0;
-    {
-        const long long ncell = 1ll << (3 * nLevels);
-        const long long nwords = (ncell + 31) / 32;
-        CKB(cudaMalloc(&childBits, nwords * 4));
-        if (vtype == VT_U8) k_leaf<1><<<grid_for(nwords), 256, 0, s>>>(dev_vol, dims[0], dims[1], dims[2], iso, childBits, nwords);
-        else k_leaf<0><<<grid_for(nwords), 256, 0, s>>>(dev_vol, dims[0], dims[1], dims[2], iso, childBits, nwords);
-        CKB(cudaGetLastError());
-        if ((st = encode(childBits, nwords, 1ull << (3 * nLevels), s, &childRanges, &childN)) != VT_OK) goto done;
-        levels[nLevels].resize(childN);
-        if (childN) CKB(cudaMemcpyAsync(levels[nLevels].data(), childRanges, childN * 8, cudaMemcpyDeviceToHost, s));
-        CKB(cudaStreamSynchronize(s));
+    /* one device allocation: every level's bits and counts, and the window */
+    Level L[14];
+    unsigned long long total[15];
+    unsigned char* ws = nullptr;
+    uint64_t* window = nullptr;
+    std::unique_ptr<uint64_t[]> host;
+    FILE* f = nullptr;
+    size_t bytes = 256;
+    for (int pass = 0; pass < 2; pass++) {
+        bytes = 256;   /* the totals */
+        for (int l = 1; l <= nLevels; l++) {
+            L[l].words = ((1ll << (3 * l)) + 31) / 32;
+            L[l].blocks = (L[l].words + CB_WORDS - 1) / CB_WORDS;
+            const size_t w4 = ((size_t)L[l].words * 4 + 255) & ~(size_t)255;
+            L[l].bits = (uint32_t*)(ws + bytes); bytes += w4;
+            L[l].offs = (uint32_t*)(ws + bytes); bytes += w4;
+            L[l].block = (unsigned long long*)(ws + bytes); bytes += ((size_t)L[l].blocks * 8 + 255) & ~(size_t)255;
+            L[l].total = (unsigned long long*)ws + l;
+        }
+        window = (uint64_t*)(ws + bytes); bytes += (size_t)RANGE_WINDOW * 8;
+        if (pass == 0) CKB(cudaMalloc(&ws, bytes));
     }
-    for (int l = nLevels - 1; l >= 1; l--) {
-        const long long np = 1ll << (3 * l);
-        const long long nwords = (np + 31) / 32;
-        uint32_t* bits = nullptr;
-        uint64_t* ranges = nullptr;
-        long long n = 0;
-        CKB(cudaMalloc(&bits, nwords * 4));
-        k_inner<<<grid_for(nwords), 256, 0, s>>>(childBits, childRanges, childN, 1ull << (3 * l), (uint64_t)(np - 1),
-                                                 bits, nwords, np);
-        CKB(cudaGetLastError());
-        st = encode(bits, nwords, 1ull << (3 * l), s, &ranges, &n);
-        cudaFree(childBits);
-        cudaFree(childRanges);
-        childBits = bits;
-        childRanges = ranges;
-        childN = n;
-        if (st != VT_OK) goto done;
-        levels[l].resize(n);
-        if (n) CKB(cudaMemcpyAsync(levels[l].data(), ranges, n * 8, cudaMemcpyDeviceToHost, s));
-        CKB(cudaStreamSynchronize(s));
-    }
-    /* root (src/CreateOctree.cu:532-540) */
-    if (vtsearch::search_children_host(levels[1].data(), (int64_t)levels[1].size(), 1ull) > 0) levels[0] = {1ull, 1ull};
     {
-        FILE* f = fopen(out_path, "wb");
+        /* cells outside the volume have no corner inside it: their words stay 0 */
+        CKB(cudaMemsetAsync(L[nLevels].bits, 0, (size_t)L[nLevels].words * 4, s));
+        const long long nbx = (dims[0] + LB_X - 1) / LB_X, nby = (dims[1] + LB_Y - 1) / LB_Y, nbz = (dims[2] + LB_Z - 1) / LB_Z;
+        const long long boxes = nbx * nby * nbz;
+        const unsigned int grid = (unsigned int)(boxes < 148 * 64 ? (boxes < 1 ? 1 : boxes) : 148 * 64);
+        if (vtype == VT_U8) k_leaf<1><<<grid, 256, 0, s>>>(dev_vol, dims[0], dims[1], dims[2], iso, L[nLevels].bits, dimension, nby, nbz, boxes);
+        else k_leaf<0><<<grid, 256, 0, s>>>(dev_vol, dims[0], dims[1], dims[2], iso, L[nLevels].bits, dimension, nby, nbz, boxes);
+        CKB(cudaGetLastError());
+    }
+    for (int l = nLevels; l >= 1; l--) {
+        if (l < nLevels)
+            k_inner<<<grid_for(L[l].words * 32, 256), 256, 0, s>>>(L[l + 1], L[l].bits, L[l].words, 1ll << (3 * l));
+        k_count<<<grid_for(L[l].blocks * 256, 256), 256, 0, s>>>(L[l]);
+        k_scan<<<1, 1024, 0, s>>>(L[l]);
+        CKB(cudaGetLastError());
+    }
+    CKB(cudaMemcpyAsync(total, ws, (size_t)(nLevels + 1) * 8, cudaMemcpyDeviceToHost, s));
+    CKB(cudaMemcpyAsync(&total[14], L[1].bits, 4, cudaMemcpyDeviceToHost, s));
+    CKB(cudaStreamSynchronize(s));
+    for (int l = nLevels; l >= 1; l--)
+        if (2 * total[l] > 0x7FFFFFFFull) { st = vtrt::fail(VT_ERR_UNSUPPORTED, "level with %llu ranges exceeds the file format", total[l]); goto done; }
+    {
+        f = fopen(out_path, "wb");
         if (!f) { st = vtrt::fail(VT_ERR_IO, "unable to write %s", out_path); goto done; }
         int magic = 919278872;
         bool ok = fwrite(&magic, 4, 1, f) == 1 && fwrite(&iso, 4, 1, f) == 1 && fwrite(&dimension, 4, 1, f) == 1 &&
                   fwrite(rd, 4, 3, f) == 3 && fwrite(&nLevels, 4, 1, f) == 1;
-        for (int l = nLevels; ok && l >= 0; l--) {
-            int n = (int)levels[l].size();
-            ok = fwrite(&n, 4, 1, f) == 1 && (n == 0 || fwrite(levels[l].data(), 8, (size_t)n, f) == (size_t)n);
+        host.reset(new uint64_t[RANGE_WINDOW]);
+        long long next = 0;   /* of level l */
+        for (int l = nLevels; ok && l >= 1;) {
+            /* as much of the following levels as the window holds */
+            struct { int l; long long k0, k1; } seg[16];
+            int n = 0;
+            long long fill = 0;
+            while (l >= 1 && fill < RANGE_WINDOW && n < 16) {
+                const long long words = (long long)(2 * total[l]), k1 = std::min(words, next + RANGE_WINDOW - fill);
+                seg[n].l = l; seg[n].k0 = next; seg[n].k1 = k1; n++;
+                if (k1 > next)
+                    k_ranges<<<grid_for(L[l].words, 256), 256, 0, s>>>(L[l], 1ull << (3 * l), (unsigned long long)next,
+                                                                       (unsigned long long)k1, window + fill);
+                fill += k1 - next;
+                next = k1;
+                if (next == words) { l--; next = 0; }
+            }
+            CKB(cudaGetLastError());
+            if (fill) CKB(cudaMemcpyAsync(host.get(), window, (size_t)fill * 8, cudaMemcpyDeviceToHost, s));
+            CKB(cudaStreamSynchronize(s));
+            const uint64_t* e = host.get();
+            for (int i = 0; ok && i < n; i++) {
+                const int words = (int)(2 * total[seg[i].l]);
+                const size_t m = (size_t)(seg[i].k1 - seg[i].k0);
+                ok = (seg[i].k0 > 0 || fwrite(&words, 4, 1, f) == 1) && (m == 0 || fwrite(e, 8, m, f) == m);
+                e += m;
+            }
         }
+        /* root (src/CreateOctree.cu:532-540), from level 1's eight bits */
+        uint64_t e1[8], root[2] = {1ull, 1ull};
+        int n1 = 0;
+        const uint32_t m1 = (uint32_t)total[14] & 0xFFu;
+        for (int k = 0; k < 8; k++) {
+            if (!((m1 >> k) & 1u)) continue;
+            if (k == 0 || !((m1 >> (k - 1)) & 1u)) e1[n1++] = 8ull + k;
+            if (k == 7 || !((m1 >> (k + 1)) & 1u)) e1[n1++] = 8ull + k;
+        }
+        const int n0 = vtsearch::search_children_host(e1, n1, 1ull) > 0 ? 2 : 0;
+        ok = ok && fwrite(&n0, 4, 1, f) == 1 && (n0 == 0 || fwrite(root, 8, 2, f) == 2);
         if (fclose(f) != 0) ok = false;
+        f = nullptr;
         if (!ok) st = vtrt::fail(VT_ERR_IO, "short write to %s", out_path);
     }
 done:
-    cudaFree(childBits);
-    cudaFree(childRanges);
+    if (f) fclose(f);
+    cudaFree(ws);
     return st;
 }
 

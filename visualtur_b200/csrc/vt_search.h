@@ -104,4 +104,40 @@ VT_SHD int search_children_host(const uint64_t* e, int64_t n, uint64_t father) {
     return num;
 }
 
+/* The same searches by rank.  A level's ranges are its runs of set codes, so
+ * where a code lies among them is known from a count: `rank` = runs that
+ * start at or before it, and whether it is set (`inside`: it lies in run
+ * rank - 1).  Every comparison of closer_host follows from these two, and
+ * the search needs no range. */
+VT_SHD int64_t closer_rank(int64_t rank, bool inside, int64_t lo, int64_t hi) {
+    for (;;) {
+        const int64_t diff = hi - lo;
+        int64_t mid = lo + diff / 2;
+        if (mid % 2 == 1) mid--;
+        if (diff <= 1) return mid;
+        const int64_t q = mid / 2;                   /* the run at e[mid], e[mid + 1] */
+        if (inside && q == rank - 1) return mid;
+        if (q >= rank) hi = mid - 1;                 /* c < e[mid] */
+        else lo = mid + 2;                           /* c > e[mid + 1] */
+    }
+}
+/* search_children_host(...) > 0 for a father whose children are the bits of
+ * `byte` at its level's codes: n = 2 * runs of the level, before = runs that
+ * start before the first child, starts = the children that start a run */
+VT_SHD bool has_children_rank(int64_t n, unsigned int byte, unsigned int starts, int64_t before) {
+    if (n <= 0 || !byte) return false;
+    if (n == 2) return true;
+    int64_t rank = before;
+    int64_t r[8];
+    for (int k = 0; k < 8; k++) { rank += (starts >> k) & 1u; r[k] = rank; }
+    const int64_t w0 = closer_rank(r[0], byte & 1u, 0, n);
+    int64_t w1 = closer_rank(r[7], (byte >> 7) & 1u, w0, n) + 1;
+    if (w1 >= n) w1 = n - 1;
+    for (int k = 0; k < 8; k++) {
+        const int64_t i = 2 * (r[k] - 1);
+        if (((byte >> k) & 1u) && i >= w0 && i < w1) return true;
+    }
+    return false;
+}
+
 }  // namespace vtsearch
