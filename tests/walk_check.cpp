@@ -72,7 +72,7 @@ static void literal(const Tree& t, const RayInv& r, unsigned node, int level, in
 static int walk(const Tree& t, const RayInv& r, std::mt19937& g, std::vector<Cand>& out) {
     Tree64 T = {t.t64.data(), t.nLevels, t.Lo};
     Walk w;
-    uint2 path[VT_TREE64_LEVELS];
+    PathNode path[VT_TREE64_LEVELS];
     int s = walk_root<1>(T, r, w, path);
     if (s != WALK_CANDIDATE) return s;
     bool fresh = true;

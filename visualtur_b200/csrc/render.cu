@@ -429,7 +429,9 @@ __device__ __forceinline__ void shade_hit(const TraceArgs& A, Ray& R, const Samp
     float dif = fabsf(n.x * l.x + n.y * l.y + n.z * l.z);
     float a = X.y / 256.0f;
     R.rgba = make_float4((1 - a) * dif, a * dif, 0.0f * dif, 1.0f);
-    R.hit = true; R.node = node_code(x, y, z, A.oct.Lo); R.brick = node_code(bx, by, bz, A.oct.Lc); R.n = n;
+    R.hit = true; R.n = n;
+    if (A.out.node) R.node = node_code(x, y, z, A.oct.Lo);
+    if (A.out.brick) R.brick = node_code(bx, by, bz, A.oct.Lc);
     R.t = dot(sub(X, R.r.o), R.dir);
 }
 
@@ -559,26 +561,29 @@ __device__ void lookahead_requests(const TraceArgs& A, Ray R, Stk& st, unsigned 
     }
 }
 
-/* padded global ray index -> view and pixel (tile order) */
-__device__ __forceinline__ bool decode_ray(const DevView* sv, int nv, int tw, int th, unsigned int g, int& v, int& i,
-                                           int& j) {
+/* padded global ray index -> view and pixel (tile order); the divisions by
+ * shifts and a product where the host found them exact */
+__device__ __forceinline__ bool decode_ray(const TraceArgs& A, const DevView* sv, unsigned int g, int& v, int& i, int& j) {
     v = 0;
     for (int b = VT_MAX_VIEWS / 2; b; b >>= 1)   /* last view whose base is <= g */
-        if (v + b < nv && sv[v + b].rayBase <= g) v += b;
-    unsigned int local = g - sv[v].rayBase;
-    unsigned int tile = local / (unsigned)(tw * th), lt = local % (unsigned)(tw * th);
-    unsigned int ti = tile / sv[v].tilesX, tj = tile % sv[v].tilesX;
-    i = (int)(ti * th + lt / tw);
-    j = (int)(tj * tw + lt % tw);
+        if (v + b < A.views.n && sv[v + b].rayBase <= g) v += b;
+    const unsigned int local = g - sv[v].rayBase, tilesX = sv[v].tilesX, inv = sv[v].tilesXInv;
+    const unsigned int rays = (unsigned int)(A.tile_w * A.tile_h);
+    const bool pow2 = A.tile_shift >= 0;
+    const unsigned int tile = pow2 ? local >> A.tile_shift : local / rays, lt = local - tile * rays;
+    const unsigned int ti = inv ? __umulhi(tile, inv) : tile / tilesX, tj = tile - ti * tilesX;
+    const unsigned int li = pow2 ? lt >> A.tile_w_shift : lt / (unsigned int)A.tile_w;
+    i = (int)(ti * A.tile_h + li);
+    j = (int)(tj * A.tile_w + (lt - li * A.tile_w));
     return i < sv[v].cam.H && j < sv[v].cam.W;
 }
 
 /* ray g's camera ray; false for tile padding */
 __device__ __forceinline__ bool ray_of(const TraceArgs& A, const DevView* sv, unsigned int g, int& view, int& i, int& j,
                                        float3& dir, RayInv& r) {
-    if (!decode_ray(sv, A.views.n, A.tile_w, A.tile_h, g, view, i, j)) return false;
+    if (!decode_ray(A, sv, g, view, i, j)) return false;
     const DevCamera& C = sv[view].cam;
-    dir = ray_dir(C.look, C.up, C.right, C.dist, C.h, C.w, C.H, C.W, i, j);
+    dir = ray_dir(C.look, C.up, C.right, C.dist, C.h, C.w, C.ih, C.iw, i, j);
     r.o = C.pos; r.dx = 1 / dir.x; r.dy = 1 / dir.y; r.dz = 1 / dir.z;
     return true;
 }
@@ -709,7 +714,7 @@ __device__ __noinline__ void literal_ray(const TraceArgs& A, const DevView* sv, 
 }
 
 #define VT_TRACE_THREADS 128
-#define VT_TRACE_CTAS 7
+#define VT_TRACE_CTAS 6
 
 /* One ray of k_trace in flight. */
 struct Trip {
@@ -767,7 +772,7 @@ __device__ __forceinline__ int try_candidate(const TraceArgs& A, Trip& R, float 
  * TRIP_LITERAL, or -1 for tile padding. */
 template <bool SKIP>
 __device__ __forceinline__ int start_trip(const TraceArgs& A, const DevView* sv, const SuspRec& rec, Trip& R,
-                                          uint2* path, unsigned long long* sk) {
+                                          PathNode* path, unsigned long long* sk) {
     R.g = rec.ray;
     R.pidx = 0xFFFFFFFFu; R.slot = 0;
     R.fresh = true; R.taken = 0;
@@ -801,7 +806,7 @@ __device__ __forceinline__ int start_trip(const TraceArgs& A, const DevView* sv,
  * until a hit, an absent brick or the end of the walk.  Set-aside candidates
  * as in run_ray. */
 template <int VTYPE, bool SLAB, int U, bool SKIP>
-__device__ __forceinline__ int advance_trip(const TraceArgs& A, Trip& R, uint2* path, unsigned long long* sk,
+__device__ __forceinline__ int advance_trip(const TraceArgs& A, Trip& R, PathNode* path, unsigned long long* sk,
                                             unsigned int* cnt) {
     if (SKIP) {
         while (R.resumeSkips) {
@@ -846,7 +851,7 @@ __device__ __forceinline__ int advance_trip(const TraceArgs& A, Trip& R, uint2* 
 
 /* Speculative requests: walks on from a suspended ray's candidate (without
  * marching) and requests up to `lookahead` further absent bricks. */
-__device__ __forceinline__ void lookahead_walk(const TraceArgs& A, Trip& R, uint2* path) {
+__device__ __forceinline__ void lookahead_walk(const TraceArgs& A, Trip& R, PathNode* path) {
     const int Lo = A.oct.Lo, Lc = A.oct.Lc;
     int want = A.ctl.lookahead, budget = 256;
     unsigned int last = 0xFFFFFFFFu, entered = 0;
@@ -864,7 +869,7 @@ __device__ __forceinline__ void lookahead_walk(const TraceArgs& A, Trip& R, uint
 }
 
 template <bool SLAB, bool SKIP>
-__device__ __forceinline__ void suspend_trip(const TraceArgs& A, Trip& R, uint2* path,
+__device__ __forceinline__ void suspend_trip(const TraceArgs& A, Trip& R, PathNode* path,
                                              const unsigned long long* sk, unsigned int* cnt) {
     cnt[VT_C_SUSPENDED]++;
     unsigned int q = atomicAdd(A.ctl.n_out, 1u);
@@ -892,7 +897,7 @@ __device__ __forceinline__ void suspend_trip(const TraceArgs& A, Trip& R, uint2*
  * one together) and writes the pixel, suspends the ray, or hands it to the
  * literal search. */
 template <int VTYPE, bool SLAB, int U, bool SKIP>
-__device__ __forceinline__ void finish_trip(const TraceArgs& A, const DevView* sv, Trip& R, uint2* path,
+__device__ __forceinline__ void finish_trip(const TraceArgs& A, const DevView* sv, Trip& R, PathNode* path,
                                             const unsigned long long* sk, int s, unsigned int* cnt) {
     if (s == RAY_DONE || s == RAY_TENTATIVE || s == TRIP_MISS) {
         Ray P;
@@ -936,18 +941,19 @@ __device__ __forceinline__ void warp_counters(unsigned int* s_cnt, const unsigne
 
 /* One ray per lane, `group` rays a warp (a tile of the screen); a warp's rays
  * walk, march and, at the end, shade together.  Bound by instruction issue
- * and divergence (1920x1080 frame of the 512^3 blobs, warm: 67 % issue
- * active, 15 of 32 lanes per instruction, 356 M warp instructions) and, on
- * small frames, by the latency of the slowest warp.  Seven CTAs of 128
- * threads per SM (72 registers): 5 CTAs 651 us, 6 627, 7 617, 8 634, 10 699
- * on that frame.  Against the binary depth-first search it replaces: 767 ->
- * 608 us there, 4.18 -> 3.55 ms for 16 mixed views, 769 -> 446 us for a
- * 1277x719 uint8 frame with bisection, 94 -> 49 us for a 96x96 frame. */
+ * and divergence (1920x1080 frame of the 512^3 blobs, warm: two thirds of
+ * the issue slots, 15 of 32 lanes per instruction) and, on small frames, by
+ * the latency of the slowest warp; of an average warp's time the walk takes
+ * 57 %, the march 26 %, set-up and shading the rest.  Six CTAs of 128
+ * threads per SM (80 registers): 5 CTAs 594 us, 6 574, 7 580, 8 601 on that
+ * frame.  Against the binary depth-first search it replaced: 767 -> 562 us
+ * there, 4.18 -> 3.47 ms for 16 mixed views, 769 -> 390 us for a 1277x719
+ * uint8 frame with bisection, 94 -> 39 us for a 96x96 frame. */
 template <int VTYPE, bool SLAB, int U, bool SKIP>
 __global__ void __launch_bounds__(VT_TRACE_THREADS, VT_TRACE_CTAS) k_trace(const __grid_constant__ TraceArgs A) {
-    __shared__ uint2 s_path[VT_TREE64_LEVELS * VT_TRACE_THREADS];   /* per thread: the node entered at each level */
+    __shared__ PathNode s_path[VT_TREE64_LEVELS * VT_TRACE_THREADS];   /* per thread: the node entered at each level */
     __shared__ unsigned int s_cnt[VT_C_COUNT];
-    uint2* const path = s_path + threadIdx.x;
+    PathNode* const path = s_path + threadIdx.x;
     if (threadIdx.x < VT_C_COUNT) s_cnt[threadIdx.x] = 0;
     __syncthreads();
     const DevView* const sv = A.views.v;
@@ -1171,7 +1177,7 @@ __global__ void __launch_bounds__(128) k_wf_march(TraceArgs A, WaveRound W, unsi
         for (unsigned int k = threadIdx.x; k < count && start + k < W.items_cap; k += blockDim.x) {
             const MarchItem it = W.sorted[start + k];
             Ray R;
-            decode_ray(sv, A.views.n, A.tile_w, A.tile_h, it.g, R.view, R.i, R.j);
+            decode_ray(A, sv, it.g, R.view, R.i, R.j);
             R.g = it.g;
             R.dir = f3(it.dx, it.dy, it.dz);
             R.r.o = sv[R.view].cam.pos;
@@ -1211,7 +1217,7 @@ __global__ void k_rays(DevCamera C, float* dirs) {
     long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= (long long)C.W * C.H) return;
     int i = (int)(id / C.W), j = (int)(id % C.W);
-    float3 d = ray_dir(C.look, C.up, C.right, C.dist, C.h, C.w, C.H, C.W, i, j);
+    float3 d = ray_dir(C.look, C.up, C.right, C.dist, C.h, C.w, C.ih, C.iw, i, j);
     dirs[3 * id] = d.x; dirs[3 * id + 1] = d.y; dirs[3 * id + 2] = d.z;
 }
 
@@ -1264,7 +1270,7 @@ __global__ void k_cube(DevCamera C, const float* cube, int3 pmin, int3 cdim, int
     const int j = (int)(tile % tilesX * 8) + (lane & 7);
     if (i >= C.H || j >= C.W) return;
     const long long tid = i * C.W + j;
-    float3 ray = ray_dir(C.look, C.up, C.right, C.dist, C.h, C.w, C.H, C.W, (int)i, j);
+    float3 ray = ray_dir(C.look, C.up, C.right, C.dist, C.h, C.w, C.ih, C.iw, (int)i, j);
     RayInv r; r.o = C.pos; r.dx = 1 / ray.x; r.dy = 1 / ray.y; r.dz = 1 / ray.z;
     int3 mb = pmin;
     const int D = cdim.x + 2 * cinc.x;

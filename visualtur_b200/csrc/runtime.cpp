@@ -119,6 +119,7 @@ static DevCamera dev_camera(const vt_camera& c) {
     DevCamera d;
     d.look = mk3(c.look); d.up = mk3(c.up); d.right = mk3(c.right); d.pos = mk3(c.position);
     d.h = c.h; d.w = c.w; d.dist = c.distance; d.W = c.W; d.H = c.H;
+    d.ih = c.h / c.H; d.iw = c.w / c.W;
     return d;
 }
 
@@ -586,6 +587,10 @@ static void fill_args(vt_handle* h, TraceArgs& a, int nViews, unsigned int total
     a.iso = h->oct->iso;
     a.light = make_float3(0.0f, 512.0f, 0.0f);   /* src/visualTur.cu:30 */
     a.tile_w = h->opt.tile_w; a.tile_h = h->opt.tile_h;
+    const int rays = a.tile_w * a.tile_h;
+    const bool pow2 = !(rays & (rays - 1)) && !(a.tile_w & (a.tile_w - 1));
+    a.tile_shift = pow2 ? __builtin_ctz(rays) : -1;
+    a.tile_w_shift = pow2 ? __builtin_ctz(a.tile_w) : -1;
     a.unroll = h->opt.unroll;
     a.refine = h->opt.refine;
 }
@@ -759,7 +764,10 @@ static vt_status render_views_inner(vt_handle* h, const ViewReq* vr, int n, cuda
         v.rgba = vr[k].rgba; v.rgb8 = vr[k].rgb8;
         v.rayBase = (unsigned int)base;
         v.tilesX = (unsigned int)((c.W + tw - 1) / tw);
-        base += (unsigned long long)v.tilesX * ((c.H + th - 1) / th) * (unsigned long long)(tw * th);
+        const unsigned long long tiles = (unsigned long long)v.tilesX * ((c.H + th - 1) / th);
+        /* the product's error stays below one quotient: tiles * tilesX < 2^32 */
+        v.tilesXInv = v.tilesX > 1 && tiles * v.tilesX < (1ull << 32) ? (unsigned int)((1ull << 32) / v.tilesX + 1) : 0u;
+        base += tiles * (unsigned long long)(tw * th);
         real += (unsigned long long)c.W * c.H;
     }
     if (base > 0xFFFFFFFFull) return fail(VT_ERR_UNSUPPORTED, "more than 2^32 rays in one call");

@@ -46,6 +46,9 @@ struct Walk {
     unsigned int mlo, mhi, first;   /* the node */
 };
 
+/* a node on the walk's path: its mask, first child and exit product */
+typedef uint4 PathNode;
+
 VT_HD float bits_float(int b) {
 #ifdef __CUDA_ARCH__
     return __int_as_float(b);
@@ -83,6 +86,7 @@ VT_HD unsigned int child_index(const Walk& w) {
     const unsigned int below = (1u << (w.idx & 31)) - 1u;
     return w.first + ((w.idx & 32) ? popc32(w.mlo) + popc32(w.mhi & below) : popc32(w.mlo & below));
 }
+VT_HD PathNode path_node(const Walk& w) { return make_uint4(w.mlo, w.mhi, w.first, (unsigned int)float_bits(w.Tn)); }
 VT_HD void load_node(const Tree64& T, unsigned int n, Walk& w) {
 #ifdef __CUDA_ARCH__
     const uint4 v = __ldg(T.nodes + n);
@@ -92,31 +96,24 @@ VT_HD void load_node(const Tree64& T, unsigned int n, Walk& w) {
     w.mlo = v.x; w.mhi = v.y; w.first = v.z;
 }
 
-/* One axis of entering a node of edge 4 q (two: 2 q) at product tc.  p, t:
- * the plane the ray would leave the node by on this axis and its product;
- * they become those of the cell.  k gets the cell's coordinate in the node.
- * A plane is passed when its product lies before tc; true when one equals
- * it. */
-VT_HD bool enter_axis(float q, float o, float inv, float tc, float& p, float& t, int& k, bool two = false) {
-    const bool pos = inv >= 0;
-    const float sq = pos ? q : -q;
-    float pm = p, tm = t;
-    bool passed = true, tie = false;
+/* One axis of entering a node of edge 4 q (two: 2 q) at product tc, sq = q
+ * with the ray's sign.  p, t: the plane the ray would leave the node by on
+ * this axis and its product; they become those of the cell.  Returns the
+ * number of cells behind it.  A plane is passed when its product lies before
+ * tc; one that equals it becomes the cell's exit plane, and the walk's next
+ * look at the cell (which must end after tc) finds the tie. */
+VT_HD int enter_axis(float sq, float o, float inv, float tc, float& p, float& t, bool two) {
+    float b = p, bt = t;          /* far plane of the half the ray is in */
+    bool far = !two;              /* it is the second half */
     if (!two) {
-        pm = p - 2 * sq;
-        tm = plane_t(pm, o, inv);
-        passed = tm < tc;
-        tie = tm == tc;
+        const float pm = p - 2 * sq, tm = plane_t(pm, o, inv);
+        far = tm < tc;
+        if (!far) { b = pm; bt = tm; }
     }
-    /* the quarter plane of the half the ray is in */
-    const float pq = passed ? p - sq : pm - sq, tq = plane_t(pq, o, inv);
-    const bool pqd = tq < tc;
-    tie |= tq == tc;
-    const int n = (passed && !two ? 2 : 0) + (pqd ? 1 : 0);   /* cells behind it */
-    k = pos ? n : (two ? 1 : 3) - n;
-    if (!pqd) { p = pq; t = tq; }
-    else if (!passed) { p = pm; t = tm; }
-    return tie;
+    const float pq = b - sq, tq = plane_t(pq, o, inv);
+    const bool passed = tq < tc;
+    p = passed ? b : pq; t = passed ? bt : tq;
+    return (far ? 2 : 0) + (passed ? 1 : 0);
 }
 
 VT_HD bool finite_f(float v) { return v - v == 0.0f; }
@@ -135,31 +132,35 @@ VT_HD bool root_span(const Tree64& T, const RayInv& r, Walk& w) {
     return finite_f(ax) && finite_f(bx) && finite_f(ay) && finite_f(by) && finite_f(az) && finite_f(bz);
 }
 
+/* the mask bits of the axes the ray runs down on (flips a cell counted along
+ * the ray into its mask bit, within a node of `two` or four cells an axis) */
+VT_HD int flip_bits(const RayInv& r, bool two) {
+    return ((r.dx >= 0 ? 0 : 48) | (r.dy >= 0 ? 0 : 12) | (r.dz >= 0 ? 0 : 3)) & (two ? 21 : 63);
+}
 /* into node n (cells of edge 1 << w.sh) at product w.tc */
 template <int STRIDE>
-VT_HD bool enter_node(const Tree64& T, const RayInv& r, Walk& w, uint2* path, unsigned int n, bool two = false) {
+VT_HD void enter_node(const Tree64& T, const RayInv& r, Walk& w, PathNode* path, unsigned int n, bool two = false) {
     const int shS = T.nLevels - T.Lo;
-    path[((w.sh - shS) >> 1) * STRIDE] = make_uint2(n, (unsigned int)float_bits(w.Tn));
     load_node(T, n, w);
+    path[((w.sh - shS) >> 1) * STRIDE] = path_node(w);
     const float q = to_float(1 << w.sh);
-    int kx, ky, kz;
-    bool tie = enter_axis(q, r.o.x, r.dx, w.tc, w.px, w.tx, kx, two);
-    tie |= enter_axis(q, r.o.y, r.dy, w.tc, w.py, w.ty, ky, two);
-    tie |= enter_axis(q, r.o.z, r.dz, w.tc, w.pz, w.tz, kz, two);
-    w.idx = (kx << 4) | (ky << 2) | kz;
-    return tie;
+    const int nx = enter_axis(r.dx >= 0 ? q : -q, r.o.x, r.dx, w.tc, w.px, w.tx, two);
+    const int ny = enter_axis(r.dy >= 0 ? q : -q, r.o.y, r.dy, w.tc, w.py, w.ty, two);
+    const int nz = enter_axis(r.dz >= 0 ? q : -q, r.o.z, r.dz, w.tc, w.pz, w.tz, two);
+    w.idx = ((nx << 4) | (ny << 2) | nz) ^ flip_bits(r, two);
 }
 
 /* Puts the ray into the volume's first cell.  WALK_CANDIDATE: there;
  * WALK_END: it misses the volume (or the volume lies behind it). */
 template <int STRIDE>
-VT_HD int walk_root(const Tree64& T, const RayInv& r, Walk& w, uint2* path) {
+VT_HD int walk_root(const Tree64& T, const RayInv& r, Walk& w, PathNode* path) {
     if (!root_span(T, r, w)) return WALK_TIE;
     if (w.tc > w.T1 || w.T1 < 0.0f) return WALK_END;
     if (w.tc == w.T1) return WALK_TIE;
     w.Tn = w.T1;
     w.sh = T.nLevels - T.Lo + 2 * (((T.Lo + 1) >> 1) - 1);
-    return enter_node<STRIDE>(T, r, w, path, 0, T.Lo & 1) ? WALK_TIE : WALK_CANDIDATE;
+    enter_node<STRIDE>(T, r, w, path, 0, T.Lo & 1);
+    return WALK_CANDIDATE;
 }
 
 /* low corner of the current cell on an axis */
@@ -174,7 +175,7 @@ VT_HD void walk_cell(const Tree64& T, const RayInv& r, const Walk& w, int& x, in
 /* Puts the ray back into candidate cell (x,y,z), as it was when the walk
  * yielded it. */
 template <int STRIDE>
-VT_HD void walk_at(const Tree64& T, const RayInv& r, int x, int y, int z, Walk& w, uint2* path) {
+VT_HD void walk_at(const Tree64& T, const RayInv& r, int x, int y, int z, Walk& w, PathNode* path) {
     const int shS = T.nLevels - T.Lo;
     const bool sx = r.dx >= 0, sy = r.dy >= 0, sz = r.dz >= 0;
     root_span(T, r, w);
@@ -182,8 +183,8 @@ VT_HD void walk_at(const Tree64& T, const RayInv& r, int x, int y, int z, Walk& 
     unsigned int n = 0;
     float ex = 0, ey = 0, ez = 0;
     for (int k = ((T.Lo + 1) >> 1) - 1; k >= 0; k--) {
-        path[k * STRIDE] = make_uint2(n, (unsigned int)float_bits(w.Tn));
         load_node(T, n, w);
+        path[k * STRIDE] = path_node(w);
         w.sh = shS + 2 * k;
         const int cx = x >> (2 * k), cy = y >> (2 * k), cz = z >> (2 * k);
         w.idx = ((cx & 3) << 4) | ((cy & 3) << 2) | (cz & 3);
@@ -202,10 +203,15 @@ VT_HD void walk_at(const Tree64& T, const RayInv& r, int x, int y, int z, Walk& 
  *
  * The inner loop steps through a node's cells by the products alone: it
  * leaves the node where the next product is the node's own exit product,
- * and two planes crossed at once show as a step that does not advance.
+ * and two planes crossed at once show as a step that does not advance.  It
+ * runs until it must leave or enter a node: a warp pays for a turn of the
+ * outer loop whatever few lanes need it, so the more cheap steps before one
+ * the better (at most 1, 2, 3, 4 steps a turn: 1047, 793, 708, 654 us on a
+ * 1920x1080 frame, unbounded 584), and a node left for a set cell is
+ * followed by entering that cell in the same turn (612 -> 584 us).
  */
 template <int STRIDE>
-VT_HD int walk_next(const Tree64& T, const RayInv& r, Walk& w, uint2* path, bool fresh, int& budget, float* tf,
+VT_HD int walk_next(const Tree64& T, const RayInv& r, Walk& w, PathNode* path, bool fresh, int& budget, float* tf,
                     unsigned int* entered) {
     const int shS = T.nLevels - T.Lo;
     const bool sx = r.dx >= 0, sy = r.dy >= 0, sz = r.dz >= 0;
@@ -224,49 +230,58 @@ VT_HD int walk_next(const Tree64& T, const RayInv& r, Walk& w, uint2* path, bool
             set = m >= 0.0f && cell_set(w);
         }
         fresh = true;
-        const bool ax = w.tx == m, ay = w.ty == m, az = w.tz == m;
-        /* two planes at once: seen here where the next step would not show
-         * it, on leaving the node, and at t = 0, where the cells before and
-         * behind sort alike (their tnear is clamped to 0) */
-        const bool edge = (ax && ay) || (ax && az) || (ay && az);
-        if (!(m > w.tc) || (edge && (!set || m == 0.0f))) {
+        if (!(m > w.tc)) {
             res = WALK_TIE;
-        } else if (!set) {
-            /* out of the node: up to the one in which the plane separates two cells */
-            const int P = to_int(ax ? w.px : ay ? w.py : w.pz);
-            if (m >= w.T1) {
-                res = WALK_END;
-            } else {
-                int X = cell_low(w.px, r.dx, w.sh), Y = cell_low(w.py, r.dy, w.sh), Z = cell_low(w.pz, r.dz, w.sh);
+        } else if (!set || m == 0.0f) {
+            /* two planes at once: seen here where the next step would not
+             * show it, on leaving the node, and at t = 0, where the cells
+             * before and behind sort alike (their tnear is clamped to 0) */
+            const bool ax = w.tx == m, ay = w.ty == m, az = w.tz == m;
+            if ((ax && ay) || (ax && az) || (ay && az)) {
+                res = WALK_TIE;
+            } else if (!set) {
+                if (m >= w.T1) {
+                    res = WALK_END;
+                } else {
+                    /* out of the node: up to the one in which the plane separates two cells */
+                    const int P = to_int(ax ? w.px : ay ? w.py : w.pz);
+                    int X = cell_low(w.px, r.dx, w.sh), Y = cell_low(w.py, r.dy, w.sh), Z = cell_low(w.pz, r.dz, w.sh);
 #ifdef __CUDA_ARCH__
-                const int b = 31 - __clz(P & -P);
+                    const int b = 31 - __clz(P & -P);
 #else
-                const int b = __builtin_ctz(P);
+                    const int b = __builtin_ctz(P);
 #endif
-                w.sh = shS + ((b - shS) & ~1);
-                const int Q = 1 << w.sh;
-                X = (ax ? (sx ? P : P - Q) : X) & -Q;
-                Y = (ay ? (sy ? P : P - Q) : Y) & -Q;
-                Z = (az ? (sz ? P : P - Q) : Z) & -Q;
-                const uint2 e = path[((w.sh - shS) >> 1) * STRIDE];
-                w.Tn = bits_float((int)e.y);
-                load_node(T, e.x, w);
-                w.idx = (((X >> w.sh) & 3) << 4) | (((Y >> w.sh) & 3) << 2) | ((Z >> w.sh) & 3);
-                w.px = to_float(sx ? X + Q : X); w.py = to_float(sy ? Y + Q : Y); w.pz = to_float(sz ? Z + Q : Z);
-                w.tx = plane_t(w.px, r.o.x, r.dx); w.ty = plane_t(w.py, r.o.y, r.dy); w.tz = plane_t(w.pz, r.o.z, r.dz);
-                w.tc = m;
+                    w.sh = shS + ((b - shS) & ~1);
+                    const int Q = 1 << w.sh;
+                    X = (ax ? (sx ? P : P - Q) : X) & -Q;
+                    Y = (ay ? (sy ? P : P - Q) : Y) & -Q;
+                    Z = (az ? (sz ? P : P - Q) : Z) & -Q;
+                    const PathNode e = path[((w.sh - shS) >> 1) * STRIDE];
+                    w.mlo = e.x; w.mhi = e.y; w.first = e.z;
+                    w.Tn = bits_float((int)e.w);
+                    w.idx = (((X >> w.sh) & 3) << 4) | (((Y >> w.sh) & 3) << 2) | ((Z >> w.sh) & 3);
+                    w.px = to_float(sx ? X + Q : X); w.py = to_float(sy ? Y + Q : Y); w.pz = to_float(sz ? Z + Q : Z);
+                    w.tx = plane_t(w.px, r.o.x, r.dx); w.ty = plane_t(w.py, r.o.y, r.dy); w.tz = plane_t(w.pz, r.o.z, r.dz);
+                    w.tc = m;
+                    /* a set cell is entered in this same turn (one that ends at 0 gets the look above first) */
+                    m = fminf(fminf(w.tx, w.ty), w.tz);
+                    set = m > 0.0f && m > w.tc && cell_set(w);
+                }
             }
-        } else if (w.sh == shS) {
-            *tf = m;
-            res = WALK_CANDIDATE;
-        } else if (budget-- <= 0) {
-            res = WALK_MORE;
-        } else {
-            (*entered)++;
-            const unsigned int n = child_index(w);
-            w.sh -= 2;
-            w.Tn = m;
-            if (enter_node<STRIDE>(T, r, w, path, n)) res = WALK_TIE;
+        }
+        if (res < 0 && set) {
+            if (w.sh == shS) {
+                *tf = m;
+                res = WALK_CANDIDATE;
+            } else if (budget-- <= 0) {
+                res = WALK_MORE;
+            } else {
+                (*entered)++;
+                const unsigned int n = child_index(w);
+                w.sh -= 2;
+                w.Tn = m;
+                enter_node<STRIDE>(T, r, w, path, n);
+            }
         }
     } while (res < 0);
     return res;

@@ -33,6 +33,7 @@ struct DevCamera {
     float3 look, up, right, pos;
     float h, w, dist;
     int W, H;
+    float ih, iw;          /* h / H, w / W */
 };
 
 /* Flattened octree: records of the reachable nodes of levels 0..Lo-1 in
@@ -85,6 +86,7 @@ struct DevView {
     uint8_t* rgb8;
     unsigned int rayBase;
     unsigned int tilesX;
+    unsigned int tilesXInv; /* floor(2^32 / tilesX) + 1 where tile / tilesX is the high word of a product with it, else 0 */
 };
 struct DevViews {
     const DevView* v;
@@ -132,6 +134,7 @@ struct TraceArgs {
     float iso;
     float3 light;
     int tile_w, tile_h;
+    int tile_shift, tile_w_shift;               /* log2 of tile_w * tile_h and tile_w; -1: not powers of two */
     unsigned int group;                         /* rays a warp takes (32 or, where they are few, less) */
     int unroll;                                 /* march samples fetched per round: 1, 2, 4, 8 */
     int refine;                                 /* bisection steps before the linear refinement */

@@ -26,10 +26,10 @@ VT_HD float3 cross(float3 a, float3 b) {
 }
 VT_HD float3 normalize(float3 v) { float inv = 1.0f / sqrtf(dot(v, v)); return mul(v, inv); }
 
-/* Pixel direction of cuda_updateRays (src/Camera.cu:59-72); i = row. */
-VT_HD float3 ray_dir(float3 look, float3 up, float3 right, float distance, float h, float w, int H,
-                     int W, int i, int j) {
-    float ih = h / H, iw = w / W;
+/* Pixel direction of cuda_updateRays (src/Camera.cu:59-72); i = row; ih, iw:
+ * the pixel's extent, h / H and w / W. */
+VT_HD float3 ray_dir(float3 look, float3 up, float3 right, float distance, float h, float w, float ih, float iw, int i,
+                     int j) {
     float3 A = mul(look, distance);
     A = add(A, mul(up, -(h / 2.0f) + (ih * ((float)i + 0.5f))));
     A = add(A, mul(right, -(w / 2.0f) + (iw * ((float)j + 0.5f))));
