@@ -143,7 +143,7 @@ __global__ void k_to_bf16(const float* w, __nv_bfloat16* wb, long long n, int N,
 /* ------------------------------------------------------------------------ */
 /* C[m,n] = sum_k A[m,k] B[k,n] with a fused epilogue.  One 256-thread CTA
  * per 128 x 64 output tile (and range of K).  Per 64-deep K step the tiles
- * land in one of four shared-memory stages by 16-byte cp.async (zero-filled
+ * land in one of S shared-memory stages by 16-byte cp.async (zero-filled
  * outside the matrices), in the tensor core's unswizzled core-matrix order:
  * 128-byte core matrices of eight 16-byte rows, (128 or 64) / 8 of them side
  * by side per eight k.  A row of a core matrix is eight k of one m or n
@@ -161,18 +161,26 @@ __global__ void k_to_bf16(const float* w, __nv_bfloat16* wb, long long n, int N,
  * K is deep (the 4096-deep gradient to the last hidden layer) K is split
  * over CTAs and k_dgrad_finish adds the parts in order.  Against a kernel
  * that staged scalar by scalar, one K step at a time, in 128 x 128 tiles: a
- * training step of the 12-512-512-4096 network at batch 256 1310 -> 124 us
+ * training step of the 12-512-512-4096 network at batch 256 1310 -> 102 us
  * (that kernel's 4096-deep gradient alone, on 8 CTAs, about 1 ms), a forward
- * pass of 8 poses 161 -> 29 us. */
+ * pass of 8 poses 161 -> 20 us; of that, dependent launches and up to eight
+ * K steps in flight 124 -> 102 and 29 -> 20 us. */
 #define G_THREADS 256
 #define G_M 128
 #define G_N 64
 #define G_K 64
-#define G_STAGES 4
 #define G_STAGE_BYTES ((G_M + G_N) * G_K * 2)
-#define G_SMEM (G_STAGES * G_STAGE_BYTES)
 
 __device__ unsigned int g_mma_err;
+
+/* Programmatic dependent launch: the kernels of a pass let the next one start
+ * (its set-up overlaps this one's work and end) and wait for the one before
+ * ahead of their first access to global memory; the wait ends when that
+ * grid, and so every grid before it, is complete. */
+__device__ __forceinline__ void grid_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -256,10 +264,10 @@ struct GemmArgs {
  * those of the other, from tile first[i] on */
 struct GemmGroup { GemmArgs g[3]; unsigned int first[3]; };
 
-template <int OPA, int OPB, int EPI>
+template <int OPA, int OPB, int EPI, int S>
 __global__ void __launch_bounds__(G_THREADS) k_gemm_tc(const __grid_constant__ GemmGroup P) {
     extern __shared__ __align__(1024) unsigned char g_smem[];
-    __shared__ __align__(8) unsigned long long mbar[G_STAGES];
+    __shared__ __align__(8) unsigned long long mbar[S];
     __shared__ uint32_t tslot;
     __shared__ float s_sum[G_THREADS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -268,6 +276,21 @@ __global__ void __launch_bounds__(G_THREADS) k_gemm_tc(const __grid_constant__ G
     const unsigned int nTiles = (G.N + G_N - 1) / G_N;
     const int tm = tile / nTiles, m0 = tm * G_M, n0 = (tile % nTiles) * G_N;
     const int kBeg = blockIdx.z * G.kPer, kEnd = min(G.K, kBeg + G.kPer);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tslot)), "r"(G_N));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int i = 0; i < S; i++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&mbar[i])), "r"(1));
+        asm volatile("fence.mbarrier_init.release.cluster;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem = tslot;
+    /* the launch before this one may still run until here */
+    grid_wait();
     if (EPI == EPI_HIDDEN && G.loss && tile == 0 && tid == 0) *G.loss = 0.0f;
     if (OPA == OP_F32_K && G.Xb)   /* dealt out over the row block's tiles */
         for (int e = (tile % nTiles) * G_THREADS + tid; e < G_M * G.K; e += nTiles * G_THREADS) {
@@ -277,19 +300,6 @@ __global__ void __launch_bounds__(G_THREADS) k_gemm_tc(const __grid_constant__ G
                     __float2bfloat16_rn(((const float*)G.A)[(long long)(m0 + r) * G.lda + k]);
         }
 
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tslot)), "r"(G_N));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    if (tid == 0) {
-        for (int i = 0; i < G_STAGES; i++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&mbar[i])), "r"(1));
-        asm volatile("fence.mbarrier_init.release.cluster;");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = tslot;
     /* kind::f16 instruction descriptor: FP32 accumulator, BF16 A and B, their
      * majors (0: K, 1: M or N), N / 8 and M / 16 */
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((OPA & 1) ? 1u << 15 : 0u) | ((OPB & 1) ? 1u << 16 : 0u) |
@@ -299,14 +309,14 @@ __global__ void __launch_bounds__(G_THREADS) k_gemm_tc(const __grid_constant__ G
 
     auto fill = [&](int t) {   /* K step t into its stage (an empty group past the end keeps the count) */
         if (t < nk) {
-            const uint32_t st = base + (t % G_STAGES) * G_STAGE_BYTES;
+            const uint32_t st = base + (t % S) * G_STAGE_BYTES;
             load_tile<OPA, G_M>(st, G.A, G.lda, m0, G.M, kBeg + t * G_K, kEnd);
             load_tile<OPB, G_N>(st + G_M * G_K * 2, G.B, G.ldb, n0, G.N, kBeg + t * G_K, kEnd);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     auto wait_mma = [&](int t) -> bool {   /* the MMAs of K step t have read their stage */
-        const uint32_t mb = smem_u32(&mbar[t % G_STAGES]), parity = (uint32_t)(t / G_STAGES) & 1u;
+        const uint32_t mb = smem_u32(&mbar[t % S]), parity = (uint32_t)(t / S) & 1u;
         uint32_t done = 0;
         for (long long it = 0; it < (1ll << 22) && !done; it++) {
             asm volatile("{\n\t.reg .pred P1;\n\t"
@@ -318,17 +328,17 @@ __global__ void __launch_bounds__(G_THREADS) k_gemm_tc(const __grid_constant__ G
         return done != 0;
     };
 #pragma unroll 1
-    for (int t = 0; t < G_STAGES - 1; t++) fill(t);
+    for (int t = 0; t < S - 1; t++) fill(t);
     bool ok = true;
 #pragma unroll 1
     for (int t = 0; t < nk; t++) {
-        asm volatile("cp.async.wait_group %0;" :: "n"(G_STAGES - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" :: "n"(S - 2) : "memory");
         /* the tensor core reads shared memory through the async proxy */
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;");
-            const uint32_t a = base + (t % G_STAGES) * G_STAGE_BYTES, b = a + G_M * G_K * 2;
+            const uint32_t a = base + (t % S) * G_STAGE_BYTES, b = a + G_M * G_K * 2;
 #pragma unroll
             for (int j = 0; j < G_K / 16; j++) {
                 const uint64_t da = tc_desc(a + j * 2 * (G_M / 8) * 128, (G_M / 8) * 128, 128);
@@ -341,11 +351,11 @@ __global__ void __launch_bounds__(G_THREADS) k_gemm_tc(const __grid_constant__ G
                     :: "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(accum), "r"(0), "r"(0), "r"(0), "r"(0));
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         :: "r"(smem_u32(&mbar[t % G_STAGES])));
+                         :: "r"(smem_u32(&mbar[t % S])));
         }
-        /* the stage of the step before is free once its MMAs are through */
-        if (t > 0) ok = wait_mma(t - 1) && ok;
-        fill(t + G_STAGES - 1);
+        /* the next step to load takes the stage of the step before, once its MMAs are through */
+        if (t > 0 && t + S - 1 < nk) ok = wait_mma(t - 1) && ok;
+        fill(t + S - 1);
     }
     if (nk > 0) ok = wait_mma(nk - 1) && ok;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -438,6 +448,7 @@ __global__ void __launch_bounds__(256) k_dgrad_finish(const float* __restrict__ 
                                                       __nv_bfloat16* __restrict__ dz, int ldz, float* __restrict__ cs) {
     __shared__ float s[4][64];
     const int c = threadIdx.x & 63, q = threadIdx.x >> 6, n = blockIdx.x * 64 + c;
+    grid_wait();
     float sum = 0.0f;
     if (n < N) {
         float d[4] = {}, a[4] = {};
@@ -478,6 +489,7 @@ struct UpdateArgs {
 __global__ void __launch_bounds__(256) k_update(const __grid_constant__ UpdateArgs U) {
     int k = 0;
     while (k < 5 && blockIdx.x >= U.first[k + 1]) k++;
+    grid_wait();
     const long long i0 = (long long)(blockIdx.x - U.first[k]) * 256 + threadIdx.x;
     if (k >= 3) {
         const int l = k - 3, i = (int)i0, N = U.N[l];
@@ -517,11 +529,29 @@ __global__ void __launch_bounds__(256) k_update(const __grid_constant__ UpdateAr
 
 static unsigned int g1(long long n) { long long b = (n + 255) / 256; return (unsigned int)(b > 4096 ? 4096 : (b < 1 ? 1 : b)); }
 
+/* a launch that may start before the one ahead of it in the stream is done
+ * (its kernel calls grid_wait) */
+template <class... P, class... A>
+static cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c;
+    memset(&c, 0, sizeof(c));
+    c.gridDim = grid; c.blockDim = dim3(threads); c.dynamicSmemBytes = smem; c.stream = s;
+    c.attrs = &at; c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 /* n products of one kind (n > 1: parts = 1) */
 template <int OPA, int OPB, int EPI>
 static cudaError_t gemm_tc(const GemmArgs* g, int n, int parts, cudaStream_t s) {
+    /* the weight gradients make two CTAs an SM of four K steps at a usual
+     * batch; the rest one CTA of up to eight, all of them in flight at once */
+    constexpr int S = EPI == EPI_GRAD ? 4 : 8;
     /* per launch (a cheap host call): the attribute belongs to the current device */
-    cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<OPA, OPB, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, G_SMEM);
+    cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<OPA, OPB, EPI, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         S * G_STAGE_BYTES);
     if (e != cudaSuccess) return e;
     GemmGroup P;
     memset(&P, 0, sizeof(P));
@@ -532,8 +562,7 @@ static cudaError_t gemm_tc(const GemmArgs* g, int n, int parts, cudaStream_t s) 
         P.g[i] = g[i];
         tiles += (unsigned int)((g[i].N + G_N - 1) / G_N) * (unsigned int)((g[i].M + G_M - 1) / G_M);
     }
-    k_gemm_tc<OPA, OPB, EPI><<<dim3(tiles, 1, parts), G_THREADS, G_SMEM, s>>>(P);
-    return cudaGetLastError();
+    return launch_pdl(k_gemm_tc<OPA, OPB, EPI, S>, dim3(tiles, 1, parts), G_THREADS, S * G_STAGE_BYTES, s, P);
 }
 /* K parts of a product with few tiles: enough to give every SM one, each at
  * least two K steps deep */
@@ -735,8 +764,8 @@ static vt_status train_tc(vt_mlp* m, const float* x, const float* y, int batch, 
         g.C = m->part;
         const int parts = k_parts(g.M, g.N, g.K, &g.kPer);
         CKM((gemm_tc<OP_BF16_K, OP_BF16_K, EPI_PART>(&g, 1, parts, s)));
-        k_dgrad_finish<<<dim3((d[l] + 63) / 64, (batch + 15) / 16), 256, 0, s>>>(m->part, parts, m->ha[l], batch, d[l],
-                                                                               m->dz[l], m->ld[l], m->cs[l]);
+        CKM(launch_pdl(k_dgrad_finish, dim3((d[l] + 63) / 64, (batch + 15) / 16), 256, 0, s, m->part, parts, m->ha[l],
+                       batch, d[l], m->dz[l], m->ld[l], m->cs[l]));
     }
     GemmArgs g[3];
     UpdateArgs u;
@@ -762,8 +791,7 @@ static vt_status train_tc(vt_mlp* m, const float* x, const float* y, int batch, 
         blocks += (unsigned int)(d[l + 1] + 255) / 256;
     }
     if (adam) { u.adam = *adam; u.step = 1; }
-    k_update<<<blocks, 256, 0, s>>>(u);
-    CKM(cudaGetLastError());
+    CKM(launch_pdl(k_update, dim3(blocks), 256, 0, s, u));
     return VT_OK;
 }
 
