@@ -28,6 +28,7 @@
 
 #include <algorithm>
 #include <memory>
+#include <new>
 
 #include "../../include/vt.h"
 #include "vt_math.cuh"
@@ -318,6 +319,8 @@ extern "C" vt_status vt_octree_build_device(const void* dev_vol, int vtype, cons
     CKB(cudaMemcpyAsync(total, ws, (size_t)(nLevels + 1) * 8, cudaMemcpyDeviceToHost, s));
     CKB(cudaMemcpyAsync(&total[14], L[1].bits, 4, cudaMemcpyDeviceToHost, s));
     CKB(cudaStreamSynchronize(s));
+    host.reset(new (std::nothrow) uint64_t[RANGE_WINDOW]);
+    if (!host) { st = vtrt::fail(VT_ERR_NOMEM, "octree build: host window"); goto done; }
     for (int l = nLevels; l >= 1; l--)
         if (2 * total[l] > 0x7FFFFFFFull) { st = vtrt::fail(VT_ERR_UNSUPPORTED, "level with %llu ranges exceeds the file format", total[l]); goto done; }
     {
@@ -326,7 +329,6 @@ extern "C" vt_status vt_octree_build_device(const void* dev_vol, int vtype, cons
         int magic = 919278872;
         bool ok = fwrite(&magic, 4, 1, f) == 1 && fwrite(&iso, 4, 1, f) == 1 && fwrite(&dimension, 4, 1, f) == 1 &&
                   fwrite(rd, 4, 3, f) == 3 && fwrite(&nLevels, 4, 1, f) == 1;
-        host.reset(new uint64_t[RANGE_WINDOW]);
         long long next = 0;   /* of level l */
         for (int l = nLevels; ok && l >= 1;) {
             /* as much of the following levels as the window holds */
