@@ -713,8 +713,8 @@ __device__ __noinline__ void literal_ray(const TraceArgs& A, const DevView* sv, 
     }
 }
 
-#define VT_TRACE_THREADS 128
-#define VT_TRACE_CTAS 6
+#define VT_TRACE_THREADS 32
+#define VT_TRACE_CTAS 24
 
 /* One ray of k_trace in flight. */
 struct Trip {
@@ -944,11 +944,14 @@ __device__ __forceinline__ void warp_counters(unsigned int* s_cnt, const unsigne
  * and divergence (1920x1080 frame of the 512^3 blobs, warm: two thirds of
  * the issue slots, 15 of 32 lanes per instruction) and, on small frames, by
  * the latency of the slowest warp; of an average warp's time the walk takes
- * 57 %, the march 26 %, set-up and shading the rest.  Six CTAs of 128
- * threads per SM (80 registers): 5 CTAs 594 us, 6 574, 7 580, 8 601 on that
- * frame.  Against the binary depth-first search it replaced: 767 -> 562 us
- * there, 4.18 -> 3.47 ms for 16 mixed views, 769 -> 390 us for a 1277x719
- * uint8 frame with bisection, 94 -> 39 us for a 96x96 frame. */
+ * 57 %, the march 26 %, set-up and shading the rest.  One warp a CTA, so
+ * that a warp's place is free for the next tile when its own rays are done
+ * (CTAs of 128, 64, 32 threads: 3.48, 3.37, 3.35 ms for 16 mixed views, 563,
+ * 557, 557 us for that frame), 24 of them per SM (80 registers; 20, 24, 28,
+ * 32 warps: 594, 574, 580, 601 us).  Against the binary depth-first search
+ * it replaced: 767 -> 557 us there, 4.18 -> 3.35 ms for the views, 769 -> 390
+ * us for a 1277x719 uint8 frame with bisection, 94 -> 40 us for a 96x96
+ * frame. */
 template <int VTYPE, bool SLAB, int U, bool SKIP>
 __global__ void __launch_bounds__(VT_TRACE_THREADS, VT_TRACE_CTAS) k_trace(const __grid_constant__ TraceArgs A) {
     __shared__ PathNode s_path[VT_TREE64_LEVELS * VT_TRACE_THREADS];   /* per thread: the node entered at each level */
