@@ -881,7 +881,12 @@ __device__ __forceinline__ void suspend_trip(const TraceArgs& A, Trip& R, PathNo
     rec.ray = R.g;
     if (off + depth + nsk <= A.ctl.pool_cap) {
         for (unsigned int e = 0; e < nsk; e++) A.ctl.pool_out[off + e] = sk[e];
-        if (more) A.ctl.pool_out[off + nsk] = make_entry(0, A.oct.Lo, R.cx, R.cy, R.cz);
+        if (more) {
+            /* the walk's own cell: R.cx.. is a set-aside candidate where that one's brick is absent once more */
+            int x, y, z;
+            walk_cell(A.oct.t64, R.r, R.w, x, y, z);
+            A.ctl.pool_out[off + nsk] = make_entry(0, A.oct.Lo, x, y, z);
+        }
         rec.depth = depth | (nsk << 8) | ((SKIP && R.tent ? 1u : 0u) << 11) | VT_SUSP_WALK |
                     (R.taken << VT_SUSP_TAKEN_SHIFT);
         rec.off = off;
