@@ -1,0 +1,67 @@
+"""Rays that take the literal depth-first search instead of the 64-ary walk:
+a camera inside the volume on node planes of several axes (every ray meets
+coinciding planes at t = 0), and the rays left over after wavefront rounds."""
+import numpy as np
+import pytest
+
+import visualtur_b200 as vt
+from visualtur_b200.prefetch import look_at
+
+pytestmark = pytest.mark.gpu
+
+W, H = 1920, 1080
+GENS = {  # generator, dims, its parameters, isovalue, brick edge
+    "blobs": (vt.VT_GEN_BLOBS, (512, 512, 512), (256, 5.0, 30.0, 0.5, 1.5, 0.05), 0.6, 16),
+    "fractal": (vt.VT_GEN_FRACTAL_U8, (401, 290, 333), (32, 4.95, 39.2, 200.0), 128.0, 32),
+}
+
+
+@pytest.fixture(scope="module")
+def scenes(cuda, workdir):
+    torch, out = cuda, {}
+    for name, (kind, dims, prm, iso, brick) in GENS.items():
+        vol = torch.empty(dims, dtype=torch.uint8 if name == "fractal" else torch.float32, device="cuda")
+        vt.generate_volume(kind, 1001, dims, prm, device_ptr=vol.data_ptr())
+        path = "%s/literal_%s.oct" % (workdir, name)
+        vt.build_octree_device(vol.data_ptr(), vt.VT_U8 if name == "fractal" else vt.VT_F32, dims, iso, path)
+        out[name] = (vt.FileManager.wrap(vol.cpu().numpy()), vt.Octree(path), brick)
+    return out
+
+
+INSIDE, LATTICE = (128.5, 128.25, 129.5), (128, 128, 128)
+
+
+def trace_ms(scene, pos, wavefront=0):
+    """the trace kernels' time of one frame, every brick resident: the
+    shortest of several; pos None: from outside"""
+    fm, oc, brick = scene
+    c = (np.array(fm.dims, float) - 1) / 2
+    lc = oc.nLevels - int(np.log2(brick))
+    p = vt.make_params(W=W, H=H, octreeFile=None, hdf5File=None, octreeLevel=oc.nLevels - 2, levelCubes=lc,
+                       dimCube=brick, maxElementsCache=8 ** lc, maxElementsCache_CPU=8 ** lc)
+    r = vt.visualTur(p, vt.default_options(preload=1, skip=0, lookahead=0, wavefront=wavefront), volume=fm, octree=oc)
+    to = c if pos is None else (168, 188, 218)
+    if pos is None:
+        pos = c + 1.5 * max(fm.dims) * np.array([0.6, 0.3, 0.74])
+    r.set_camera(look_at(W, H, 50.0, 30.0, np.array(pos, float), np.array(to, float)))
+    ms = []
+    for _ in range(6):
+        r.updateVisibleCubes(None)
+        s = r.stats()
+        assert s["passes"] == 1
+        ms.append(s["ms_trace_last_frame"])
+    r.close()
+    return min(ms[1:])
+
+
+@pytest.mark.parametrize("name", sorted(GENS))
+@pytest.mark.parametrize("rays", ["lattice", "waiting"])
+def test_literal_rays_cost_a_search_not_more(name, rays, scenes, cuda):
+    """The binary search over all rays of these frames takes 2.0 to 3.7 times
+    what the walk takes on a general frame; 5 leaves room for both clocks.
+    (A search that adds each ray's counters to global memory: 4.8 to 22.)"""
+    if rays == "lattice":
+        got, general = trace_ms(scenes[name], LATTICE), trace_ms(scenes[name], INSIDE)
+    else:
+        got, general = trace_ms(scenes[name], None, wavefront=1), trace_ms(scenes[name], None)
+    assert got < 5 * general
