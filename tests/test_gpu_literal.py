@@ -4,7 +4,10 @@ coinciding planes at t = 0), and the rays left over after wavefront rounds."""
 import numpy as np
 import pytest
 
+import vt_fixtures as F
 import visualtur_b200 as vt
+from oracle import oracle as orc
+from test_gpu_parity import assert_parity
 from visualtur_b200.prefetch import look_at
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +68,40 @@ def test_literal_rays_cost_a_search_not_more(name, rays, scenes, cuda):
     else:
         got, general = trace_ms(scenes[name], None, wavefront=1), trace_ms(scenes[name], None)
     assert got < 5 * general
+
+
+@pytest.mark.parametrize("name, most", [("blobs", 2.1), ("fractal", 3.1)])
+def test_camera_on_a_lattice_point_costs_no_more_than_the_binary_search(name, most, scenes, cuda):
+    """Before the walk the frame from the lattice point took 1437 and 1103 us,
+    2.02 and 2.95 times what the walk takes next to it."""
+    assert trace_ms(scenes[name], LATTICE) < most * trace_ms(scenes[name], INSIDE)
+
+
+@pytest.mark.parametrize("edge", [64, 384])     # few rays a warp, full warps (the search's own kernel)
+@pytest.mark.parametrize("mode", ["resident", "slab", "cold", "cold_skip", "wave"])
+@pytest.mark.parametrize("pos", [(64, 64, 64), (32, 60.5, 64), (64, 44, 128)])
+def test_lattice_camera_parity(pos, mode, edge, workdir, cuda):
+    """Cameras inside the volume on node planes of three and two axes, and on
+    a face of it, against the oracle."""
+    c = F.CASES["c1"]
+    vol = F.case_volume("c1")
+    path = F.case_octree("c1", workdir)
+    nb = 8 ** c["levelC"] if not mode.startswith("cold") else 40
+    p = vt.make_params(W=edge, H=edge, octreeFile=None, hdf5File=None, octreeLevel=c["levelO"], levelCubes=c["levelC"],
+                       dimCube=8, cubeInc=c["inc"], distance=c["dist"], fov_H=c["fov"], fov_W=c["fov"],
+                       maxElementsCache=nb, maxElementsCache_CPU=nb)
+    opt = vt.default_options(resident=mode == "resident", preload=0, record_hits=1, lookahead=0, max_passes=100000,
+                             skip=2 if mode == "cold_skip" else 0, wavefront=2 if mode == "wave" else 0)
+    r = vt.visualTur(p, opt, volume=vt.FileManager.wrap(vol), octree=vt.Octree(path))
+    r.camera_Move(pos)
+    rgba, rgb8 = r.render_host()
+    node, brick, t, nrm = r.debug_hits()
+    st = r.stats()
+    r.close()
+    cam = orc.Camera(edge, edge, c["dist"], c["fov"], c["fov"])
+    orc.apply_ops(cam, [("mv", pos)])
+    want = orc.render(orc.Octree(path), vol, cam, c["levelO"], c["levelC"], c["inc"])
+    assert_parity(dict(rgba=rgba, rgb8=rgb8, node=node, brick=brick, t=t, normal=nrm), want)
+    assert st["rays"] == edge * edge and st["hits"] == want["agg"]["hits"] > 0
+    if mode != "cold_skip":
+        assert st["samples"] == want["agg"]["samples"] and st["candidates"] == want["agg"]["candidates"]

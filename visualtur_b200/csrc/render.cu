@@ -681,24 +681,16 @@ __device__ __forceinline__ void flush_counters(const TraceArgs& A, unsigned int*
     }
 }
 
-/* The literal depth-first search for one ray, to its end: rays whose 64-ary
- * walk met coinciding or non-finite plane products, and rays resumed with a
- * saved stack (a wavefront round's).  Rare, so it is kept out of line: its
- * stack and its registers cost the others nothing (inlined, a 1920x1080
- * frame without such rays 602 -> 648 us).  sk: set-aside candidates of a ray
- * handed over by the walk.  s_cnt: the CTA's counters in shared memory (each
- * ray adding to the ones in global memory, a frame of such rays took 8.45 ms
- * instead of 1.33 ms). */
+/* The literal depth-first search for one ray, to its end.  sk: set-aside
+ * candidates of a ray handed over by the walk. */
 template <int VTYPE, bool SLAB, int U, bool SKIP>
-__device__ __noinline__ void literal_ray(const TraceArgs& A, const DevView* sv, SuspRec rec, int nskip,
-                                         const unsigned long long* sk, unsigned int* s_cnt) {
-    unsigned int cnt[VT_C_COUNT];
-#pragma unroll
-    for (int c = 0; c < VT_C_COUNT; c++) cnt[c] = 0;
+__device__ __forceinline__ void search_ray(const TraceArgs& A, const DevView* sv, const SuspRec& rec, int nskip,
+                                           const unsigned long long* sk, unsigned int* cnt) {
     Stk st;
     Ray R;
     int s = start_ray<SKIP>(A, sv, rec, R, st);
     if (s < 0) return;
+    if (!A.ctl.in && !rec.depth) cnt[VT_C_RAYS]++;
     if (SKIP && nskip > 0) {
         R.nskip = nskip;
         for (int e = 0; e < nskip; e++) st.sk[e] = sk[e];
@@ -710,6 +702,21 @@ __device__ __noinline__ void literal_ray(const TraceArgs& A, const DevView* sv, 
         suspend_ray<VTYPE, SLAB, SKIP>(A, R, st, cnt);
     } else if (s == RAY_SUSPENDED) suspend_ray<VTYPE, SLAB, SKIP>(A, R, st, cnt);
     else if (SKIP && s == RAY_DONE_WRITTEN) cnt[VT_C_HITS]++;   /* the tentative hit stands */
+}
+
+/* The literal search in k_trace: rays whose 64-ary walk met coinciding or
+ * non-finite plane products, and rays resumed with a saved stack.  Rare, so
+ * it is kept out of line: its stack and its registers cost the others
+ * nothing (inlined, a 1920x1080 frame without such rays 602 -> 648 us).
+ * s_cnt: the CTA's counters in shared memory (each ray adding to the ones in
+ * global memory, a frame of such rays took 8.45 ms instead of 1.33 ms). */
+template <int VTYPE, bool SLAB, int U, bool SKIP>
+__device__ __noinline__ void literal_ray(const TraceArgs& A, const DevView* sv, SuspRec rec, int nskip,
+                                         const unsigned long long* sk, unsigned int* s_cnt) {
+    unsigned int cnt[VT_C_COUNT];
+#pragma unroll
+    for (int c = 0; c < VT_C_COUNT; c++) cnt[c] = 0;
+    search_ray<VTYPE, SLAB, U, SKIP>(A, sv, rec, nskip, sk, cnt);
 #pragma unroll
     for (int c = 0; c < VT_C_COUNT; c++) {
         if (!cnt[c]) continue;
@@ -1002,6 +1009,30 @@ __global__ void __launch_bounds__(VT_TRACE_THREADS, VT_TRACE_CTAS) k_trace(const
         if (v && c == VT_C_MAXSTACK) atomicMax(&A.ctl.counters[c], (unsigned long long)v);
         else if (v) atomicAdd(&A.ctl.counters[c], (unsigned long long)v);
     }
+}
+
+/* The literal search, one ray per thread: frames whose rays all need it
+ * (TraceArgs::literal) and the rays left over after wavefront rounds.  Eight
+ * 128-thread CTAs per SM: it is bound by latency, and in k_trace, with 24
+ * warps an SM, the same frames take a fifth longer (1920x1080 from a lattice
+ * point of the 512^3 blobs 1699 -> 1292 us, of the 401x290x333 uint8 fractal
+ * 1328 -> 1035 us; the 64-ary walk next to these points: 717 and 377 us). */
+template <int VTYPE, bool SLAB, bool SKIP>
+__global__ void __launch_bounds__(128, 8) k_literal(const __grid_constant__ TraceArgs A) {
+    unsigned int cnt[VT_C_COUNT];
+#pragma unroll
+    for (int c = 0; c < VT_C_COUNT; c++) cnt[c] = 0;
+    const unsigned int nItems =
+        A.ctl.in ? (A.ctl.n_in_dev ? min(*A.ctl.n_in_dev, A.ctl.n_in) : A.ctl.n_in) : A.views.totalRays;
+    const unsigned int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w < nItems) {
+        SuspRec rec;
+        if (A.ctl.in) rec = A.ctl.in[w];
+        else { rec.ray = w; rec.depth = 0; }
+        search_ray<VTYPE, SLAB, 1, SKIP>(A, A.views.v, rec, 0, nullptr, cnt);
+    }
+    __syncwarp();
+    flush_counters(A, cnt);
 }
 
 /* ---- wavefront passes ------------------------------------------------- */
@@ -1415,6 +1446,16 @@ cudaError_t vt_launch_trace(const TraceArgs& a0, bool slabMode, cudaStream_t s) 
      * in-order traversal keeps its registers; it needs bricks (slab mode)
      * and is off while a trace is logged */
     const bool skip = slabMode && a.ctl.skip > 0 && !a.ctl.touched;
+    if (a.literal && a.group == 32) {   /* few rays are better off spread over k_trace's warps */
+        const unsigned int b = (unsigned int)((items + 127ull) / 128);
+#define VT_LITERAL(V) \
+    { if (slabMode && skip) k_literal<V, true, true><<<b, 128, 0, s>>>(a); \
+      else if (slabMode) k_literal<V, true, false><<<b, 128, 0, s>>>(a); \
+      else k_literal<V, false, false><<<b, 128, 0, s>>>(a); }
+        if (a.br.vtype == 0) VT_LITERAL(0) else VT_LITERAL(1)
+#undef VT_LITERAL
+        return cudaGetLastError();
+    }
 #define VT_LAUNCH_U(V, S, K)                                                     \
     switch (a.unroll) {                                                          \
         case 2: k_trace<V, S, 2, K><<<blocks, VT_TRACE_THREADS, 0, s>>>(a); break; \

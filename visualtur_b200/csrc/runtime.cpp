@@ -595,6 +595,22 @@ static void fill_args(vt_handle* h, TraceArgs& a, int nViews, unsigned int total
     a.refine = h->opt.refine;
 }
 
+/* The views' cameras all lie where the 64-ary walk ends at once: inside the
+ * volume on node planes, as cameras at whole coordinates often do.  A frame
+ * of such rays goes to the literal search directly. */
+static bool all_literal(const vt_handle* h, int nViews) {
+    auto set = [&](int level, int x, int y, int z) {
+        const std::vector<uint64_t>& e = h->oct->levels[level];
+        const uint64_t c = vt::node_code((uint32_t)x, (uint32_t)y, (uint32_t)z, level);
+        const size_t i = (size_t)(std::upper_bound(e.begin(), e.end(), c) - e.begin());
+        /* in a range [e[i-1], e[i]], i odd, or its last code */
+        return (i & 1) || (i > 0 && e[i - 1] == c);
+    };
+    for (int k = 0; k < nViews; k++)
+        if (!vt::ties_at_start(h->h_views[k].cam.pos, h->nLevels, h->Lo, set)) return false;
+    return true;
+}
+
 static vt_status collect_counters(vt_handle* h, cudaStream_t s) {
     CK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(CtlBlock), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -691,6 +707,7 @@ static cudaError_t launch_pass(vt_handle* h, const TraceArgs& a0, bool slabMode,
     if (e != cudaSuccess) return e;
     const int p = (rounds - 1) & 1;
     a.ctl.in = h->d_wnext[p]; a.ctl.n_in = bound; a.ctl.pool_in = h->d_wpool[p]; a.ctl.n_in_dev = &h->d_wctl[p].n_next;
+    a.literal = 1;   /* these rays have saved stacks */
     *kernels = 4 * rounds + 1;
     return vt_launch_trace(a, slabMode, s);
 }
@@ -773,6 +790,7 @@ static vt_status render_views_inner(vt_handle* h, const ViewReq* vr, int n, cuda
     if (base > 0xFFFFFFFFull) return fail(VT_ERR_UNSUPPORTED, "more than 2^32 rays in one call");
     TraceArgs a;
     fill_args(h, a, n, (unsigned int)base);
+    a.literal = all_literal(h, n);
     const bool slabMode = !h->opt.resident;
     const bool allResident = h->opt.resident || h->cache->all_resident();
     vt_status st;

@@ -48,4 +48,35 @@ inline std::vector<uint4> build_tree64(const std::vector<uint2>& bin, int Lo) {
     return out;
 }
 
+/* Whether every ray from `o` ends its walk at once (WALK_TIE): from the top
+ * node down, the walk looks at the cells that touch t = 0, and where o lies
+ * on planes of two axes or more of a node's cells, the products of these
+ * planes coincide at 0.  A cell without anything in it is left without a
+ * look inside, so such planes below it do not count.  set(level, x, y, z):
+ * whether the binary octree has that node. */
+template <class Set>
+inline bool ties_at_start(float3 o, int nLevels, int Lo, Set set) {
+    const float N = (float)(1 << nLevels), p[3] = {o.x, o.y, o.z};
+    for (int a = 0; a < 3; a++)
+        if (!(p[a] >= 0.0f && p[a] <= N)) return false;
+    for (int k = (Lo + 1) / 2 - 1; k >= 0; k--) {
+        const int sh = nLevels - Lo + 2 * k, cells = 1 << (nLevels - sh);
+        int lo[3], hi[3], planes = 0;
+        for (int a = 0; a < 3; a++) {
+            hi[a] = (int)p[a] >> sh;
+            const bool on = p[a] == (float)(hi[a] << sh);
+            planes += on;
+            lo[a] = on && hi[a] > 0 ? hi[a] - 1 : hi[a];
+            if (hi[a] >= cells) hi[a] = cells - 1;
+        }
+        if (planes >= 2) return true;
+        bool any = false;
+        for (int x = lo[0]; x <= hi[0]; x++)
+            for (int y = lo[1]; y <= hi[1]; y++)
+                for (int z = lo[2]; z <= hi[2]; z++) any = any || set(nLevels - sh, x, y, z);
+        if (!any) return false;
+    }
+    return false;
+}
+
 }  // namespace vt

@@ -136,6 +136,7 @@ struct TraceArgs {
     int tile_w, tile_h;
     int tile_shift, tile_w_shift;               /* log2 of tile_w * tile_h and tile_w; -1: not powers of two */
     unsigned int group;                         /* rays a warp takes (32 or, where they are few, less) */
+    int literal;                                /* the literal search for every ray (k_literal) */
     int unroll;                                 /* march samples fetched per round: 1, 2, 4, 8 */
     int refine;                                 /* bisection steps before the linear refinement */
 };
