@@ -447,12 +447,14 @@ __global__ void __launch_bounds__(256) k_dgrad_finish(const float* __restrict__ 
                                                       const float* __restrict__ act, int M, int N,
                                                       __nv_bfloat16* __restrict__ dz, int ldz, float* __restrict__ cs) {
     __shared__ float s[4][64];
-    const int c = threadIdx.x & 63, q = threadIdx.x >> 6, n = blockIdx.x * 64 + c;
+    /* column and row blocks in one grid dimension: the other ones end at 65535 */
+    const unsigned int cols = (unsigned int)(N + 63) / 64, rb = blockIdx.x / cols;
+    const int c = threadIdx.x & 63, q = threadIdx.x >> 6, n = (int)(blockIdx.x - rb * cols) * 64 + c;
     grid_wait();
     float sum = 0.0f;
     if (n < N) {
         float d[4] = {}, a[4] = {};
-        const int m0 = blockIdx.y * 16 + q * 4;
+        const int m0 = (int)rb * 16 + q * 4;
 #pragma unroll
         for (int j = 0; j < 4; j++)
             if (m0 + j < M) a[j] = act[(long long)(m0 + j) * N + n];
@@ -471,7 +473,7 @@ __global__ void __launch_bounds__(256) k_dgrad_finish(const float* __restrict__ 
     }
     s[q][c] = sum;
     __syncthreads();
-    if (q == 0 && n < N) cs[(long long)blockIdx.y * N + n] = (s[0][c] + s[1][c]) + (s[2][c] + s[3][c]);
+    if (q == 0 && n < N) cs[(long long)rb * N + n] = (s[0][c] + s[1][c]) + (s[2][c] + s[3][c]);
 }
 
 /* The parameters of the three layers after a backward pass: bias gradients
@@ -540,7 +542,9 @@ static cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int threads, size
     memset(&c, 0, sizeof(c));
     c.gridDim = grid; c.blockDim = dim3(threads); c.dynamicSmemBytes = smem; c.stream = s;
     c.attrs = &at; c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, P(args)...);
+    if (e != cudaSuccess) cudaGetLastError();   /* reported here: not left for the caller's next check */
+    return e;
 }
 
 /* n products of one kind (n > 1: parts = 1) */
@@ -764,8 +768,8 @@ static vt_status train_tc(vt_mlp* m, const float* x, const float* y, int batch, 
         g.C = m->part;
         const int parts = k_parts(g.M, g.N, g.K, &g.kPer);
         CKM((gemm_tc<OP_BF16_K, OP_BF16_K, EPI_PART>(&g, 1, parts, s)));
-        CKM(launch_pdl(k_dgrad_finish, dim3((d[l] + 63) / 64, (batch + 15) / 16), 256, 0, s, m->part, parts, m->ha[l],
-                       batch, d[l], m->dz[l], m->ld[l], m->cs[l]));
+        CKM(launch_pdl(k_dgrad_finish, dim3(((unsigned int)d[l] + 63) / 64 * (((unsigned int)batch + 15) / 16)), 256, 0, s,
+                       m->part, parts, m->ha[l], batch, d[l], m->dz[l], m->ld[l], m->cs[l]));
     }
     GemmArgs g[3];
     UpdateArgs u;
