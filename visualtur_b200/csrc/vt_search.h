@@ -140,4 +140,26 @@ VT_SHD bool has_children_rank(int64_t n, unsigned int byte, unsigned int starts,
     return false;
 }
 
+/* Blocks [*b0, *b1) of a level that can hold words [k0, k1) of its range
+ * array.  block[b]: runs that start before block b, total: runs of the level.
+ * Block b's starts and ends are words 2 * block[b] - 1 (the end of a run that
+ * began before it) to 2 * block[b + 1] - 1. */
+VT_SHD void window_blocks(const unsigned long long* block, int64_t blocks, unsigned long long total,
+                          unsigned long long k0, unsigned long long k1, int64_t* b0, int64_t* b1) {
+    int64_t lo = 0, hi = blocks;                     /* the first with 2 * block[b + 1] > k0 */
+    while (lo < hi) {
+        const int64_t mid = lo + (hi - lo) / 2;
+        if (2 * (mid + 1 < blocks ? block[mid + 1] : total) > k0) hi = mid;
+        else lo = mid + 1;
+    }
+    *b0 = lo;
+    hi = blocks;                                     /* the first with 2 * block[b] - 1 >= k1 */
+    while (lo < hi) {
+        const int64_t mid = lo + (hi - lo) / 2;
+        if (2 * block[mid] > k1) hi = mid;
+        else lo = mid + 1;
+    }
+    *b1 = lo;
+}
+
 }  // namespace vtsearch
