@@ -19,7 +19,7 @@
  * the count before its children and their bits alone (vt_search.h,
  * has_children_rank), so no level waits for the ranges of the one below and
  * the host is asked for nothing until all levels are done.  The ranges are
- * then made, copied back and written window by window.
+ * then made and copied back window by window, and written (octree_write.h).
  * Output is byte-identical to the reference's volumeToOctree.
  */
 #include <math.h>
@@ -31,6 +31,7 @@
 #include <new>
 
 #include "../../include/vt.h"
+#include "octree_write.h"
 #include "vt_math.cuh"
 #include "vt_runtime.h"
 #include "vt_search.h"
@@ -290,7 +291,6 @@ extern "C" vt_status vt_octree_build_device(const void* dev_vol, int vtype, cons
     unsigned char* ws = nullptr;
     uint64_t* window = nullptr;
     std::unique_ptr<uint64_t[]> host;
-    FILE* f = nullptr;
     size_t bytes = 256;
     for (int pass = 0; pass < 2; pass++) {
         bytes = 256;   /* the totals */
@@ -326,60 +326,39 @@ extern "C" vt_status vt_octree_build_device(const void* dev_vol, int vtype, cons
     CKB(cudaMemcpyAsync(total, ws, (size_t)(nLevels + 1) * 8, cudaMemcpyDeviceToHost, s));
     CKB(cudaMemcpyAsync(&total[14], L[1].bits, 4, cudaMemcpyDeviceToHost, s));
     CKB(cudaStreamSynchronize(s));
-    host.reset(new (std::nothrow) uint64_t[RANGE_WINDOW]);
-    if (!host) { st = vtrt::fail(VT_ERR_NOMEM, "octree build: host window"); goto done; }
     for (int l = nLevels; l >= 1; l--)
         if (2 * total[l] > 0x7FFFFFFFull) { st = vtrt::fail(VT_ERR_UNSUPPORTED, "level with %llu ranges exceeds the file format", total[l]); goto done; }
+    host.reset(new (std::nothrow) uint64_t[RANGE_WINDOW]);
+    if (!host) { st = vtrt::fail(VT_ERR_NOMEM, "octree build: host window"); goto done; }
     {
-        f = fopen(out_path, "wb");
-        if (!f) { st = vtrt::fail(VT_ERR_IO, "unable to write %s", out_path); goto done; }
-        int magic = 919278872;
-        bool ok = fwrite(&magic, 4, 1, f) == 1 && fwrite(&iso, 4, 1, f) == 1 && fwrite(&dimension, 4, 1, f) == 1 &&
-                  fwrite(rd, 4, 3, f) == 3 && fwrite(&nLevels, 4, 1, f) == 1;
-        long long next = 0;   /* of level l */
-        for (int l = nLevels; ok && l >= 1;) {
-            /* as much of the following levels as the window holds */
-            struct { int l; long long k0, k1; } seg[16];
-            int n = 0;
-            long long fill = 0;
-            while (l >= 1 && fill < RANGE_WINDOW && n < 16) {
-                const long long words = (long long)(2 * total[l]), k1 = std::min(words, next + RANGE_WINDOW - fill);
-                seg[n].l = l; seg[n].k0 = next; seg[n].k1 = k1; n++;
+        vtoct::Levels file;
+        file.iso = iso; file.dimension = dimension; file.nLevels = nLevels; file.bits1 = (uint32_t)total[14];
+        for (int a = 0; a < 3; a++) file.realDim[a] = rd[a];
+        for (int l = 1; l <= nLevels; l++) file.runs[l] = total[l];
+        /* as much of level l from word k0 on, and of the following levels, as the window holds */
+        auto fetch = [&](int l, size_t k0, size_t* n) -> const uint64_t* {
+            long long fill = 0, next = (long long)k0;
+            for (; l >= 1 && fill < RANGE_WINDOW; l--, next = 0) {
+                const long long k1 = std::min((long long)(2 * total[l]), next + RANGE_WINDOW - fill);
                 if (k1 > next)
                     k_ranges<<<grid_for(L[l].blocks * 256, 256), 256, 0, s>>>(L[l], 1ull << (3 * l), (unsigned long long)next,
-                                                                       (unsigned long long)k1, window + fill);
+                                                                              (unsigned long long)k1, window + fill);
                 fill += k1 - next;
-                next = k1;
-                if (next == words) { l--; next = 0; }
             }
-            CKB(cudaGetLastError());
-            if (fill) CKB(cudaMemcpyAsync(host.get(), window, (size_t)fill * 8, cudaMemcpyDeviceToHost, s));
-            CKB(cudaStreamSynchronize(s));
-            const uint64_t* e = host.get();
-            for (int i = 0; ok && i < n; i++) {
-                const int words = (int)(2 * total[seg[i].l]);
-                const size_t m = (size_t)(seg[i].k1 - seg[i].k0);
-                ok = (seg[i].k0 > 0 || fwrite(&words, 4, 1, f) == 1) && (m == 0 || fwrite(e, 8, m, f) == m);
-                e += m;
-            }
+            cudaError_t e = cudaGetLastError();
+            if (e == cudaSuccess) e = cudaMemcpyAsync(host.get(), window, (size_t)fill * 8, cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess) { st = vtrt::fail(VT_ERR_CUDA, "octree build, ranges: %s", cudaGetErrorString(e)); return nullptr; }
+            *n = (size_t)fill;
+            return host.get();
+        };
+        switch (vtoct::write_octree(out_path, file, fetch)) {
+            case vtoct::WRITE_OPEN: st = vtrt::fail(VT_ERR_IO, "unable to write %s", out_path); break;
+            case vtoct::WRITE_SHORT: st = vtrt::fail(VT_ERR_IO, "short write to %s", out_path); break;
+            default: break;   /* written, or fetch's own status */
         }
-        /* root (src/CreateOctree.cu:532-540), from level 1's eight bits */
-        uint64_t e1[8], root[2] = {1ull, 1ull};
-        int n1 = 0;
-        const uint32_t m1 = (uint32_t)total[14] & 0xFFu;
-        for (int k = 0; k < 8; k++) {
-            if (!((m1 >> k) & 1u)) continue;
-            if (k == 0 || !((m1 >> (k - 1)) & 1u)) e1[n1++] = 8ull + k;
-            if (k == 7 || !((m1 >> (k + 1)) & 1u)) e1[n1++] = 8ull + k;
-        }
-        const int n0 = vtsearch::search_children_host(e1, n1, 1ull) > 0 ? 2 : 0;
-        ok = ok && fwrite(&n0, 4, 1, f) == 1 && (n0 == 0 || fwrite(root, 8, 2, f) == 2);
-        if (fclose(f) != 0) ok = false;
-        f = nullptr;
-        if (!ok) st = vtrt::fail(VT_ERR_IO, "short write to %s", out_path);
     }
 done:
-    if (f) fclose(f);
     cudaFree(ws);
     return st;
 }
