@@ -390,6 +390,13 @@ vt_status vt_mlp_info(const vt_mlp* m, int dims[4]);
 /* FP32 master weights, layer by layer: W (in x out, row-major) then b */
 vt_status vt_mlp_get_weights(vt_mlp* m, float* host, int64_t* n);
 vt_status vt_mlp_set_weights(vt_mlp* m, const float* host, int64_t n);
+/* Every wait of the tensor-core kernels is bounded.  One that gives up leaves
+ * its product incomplete: no training step of that network changes its
+ * parameters from then on, until the next of its calls that synchronises
+ * (a step that returns its loss, gradients, get or set weights) has returned
+ * VT_ERR_TIMEOUT.  This call puts a network into that state, for tests of
+ * what follows. */
+vt_status vt_debug_mlp_timeout(vt_mlp* m);
 /* vt_mlp_forward without any allocation (no counterpart in the reference).
  * For callers that cannot allocate GPU memory where they run inference --
  * a render loop in a host that owns the device's memory budget, or a frame

@@ -146,6 +146,7 @@ _PROTOS = {
     "vt_mlp_gradients": (C.c_int, [_P, _P, _P, C.c_int, _P, C.POINTER(C.c_float)]),
     "vt_mlp_get_weights": (C.c_int, [_P, _P, C.POINTER(C.c_int64)]),
     "vt_mlp_set_weights": (C.c_int, [_P, _P, C.c_int64]),
+    "vt_debug_mlp_timeout": (C.c_int, [_P]),
     "vt_mlp_forward_noalloc": (C.c_int, [_P, _P, C.c_int, _P, _P]),
     "vt_mlp_info": (C.c_int, [_P, C.c_int * 4]),
     "vt_mlp_use_tensor_cores": (C.c_int, [_P, C.c_int]),
@@ -627,6 +628,10 @@ class MLP:
     def set_weights(self, layers):
         flat = np.concatenate([np.ascontiguousarray(a, np.float32).ravel() for wb in layers for a in wb])
         check(lib().vt_mlp_set_weights(self._h, flat.ctypes.data, flat.size))
+
+    def debug_timeout(self):
+        """The state after a bounded tensor-core wait gave up (vt_debug_mlp_timeout)."""
+        check(lib().vt_debug_mlp_timeout(self._h))
 
     def _split(self, flat):
         out, o, d = [], 0, self.dims

@@ -152,7 +152,7 @@ __global__ void k_to_bf16(const float* w, __nv_bfloat16* wb, long long n, int N,
  * thread issues four tcgen05.mma (M 128, N 64, K 16) a step into a
  * 64-column tensor-memory accumulator and commits them to the stage's
  * mbarrier, which is waited for (bounded: past the limit the kernel records
- * it in g_mma_err, frees its tensor memory and returns) before the stage is
+ * it in the network's err, frees its tensor memory and returns) before the stage is
  * filled again.  The accumulator then goes through shared memory so that
  * the epilogue's reads and writes are coalesced.
  *
@@ -170,8 +170,6 @@ __global__ void k_to_bf16(const float* w, __nv_bfloat16* wb, long long n, int N,
 #define G_N 64
 #define G_K 64
 #define G_STAGE_BYTES ((G_M + G_N) * G_K * 2)
-
-__device__ unsigned int g_mma_err;
 
 /* Programmatic dependent launch: the kernels of a pass let the next one start
  * (its set-up overlaps this one's work and end) and wait for the one before
@@ -262,7 +260,7 @@ struct GemmArgs {
 };
 /* up to three products in one launch: grid.x holds the tiles of one after
  * those of the other, from tile first[i] on */
-struct GemmGroup { GemmArgs g[3]; unsigned int first[3]; };
+struct GemmGroup { GemmArgs g[3]; unsigned int first[3]; unsigned int* err; };
 
 template <int OPA, int OPB, int EPI, int S>
 __global__ void __launch_bounds__(G_THREADS) k_gemm_tc(const __grid_constant__ GemmGroup P) {
@@ -324,7 +322,7 @@ __global__ void __launch_bounds__(G_THREADS) k_gemm_tc(const __grid_constant__ G
                          "selp.b32 %0, 1, 0, P1;\n\t}"
                          : "=r"(done) : "r"(mb), "r"(parity) : "memory");
         }
-        if (!done) atomicOr(&g_mma_err, 1u);
+        if (!done) atomicOr(P.err, 1u);
         return done != 0;
     };
 #pragma unroll 1
@@ -487,11 +485,13 @@ struct UpdateArgs {
     float *b[3], *bm[3], *bv[3], *gb[3]; const float* part[3]; int parts[3];
     unsigned int first[7];   /* blocks: weights of layer 0, 1, 2, biases of layer 0, 1, 2 */
     Adam adam; int step;
+    const unsigned int* err;   /* set: a product of this pass is incomplete, no step */
 };
 __global__ void __launch_bounds__(256) k_update(const __grid_constant__ UpdateArgs U) {
     int k = 0;
     while (k < 5 && blockIdx.x >= U.first[k + 1]) k++;
     grid_wait();
+    if (U.step && *U.err) return;
     const long long i0 = (long long)(blockIdx.x - U.first[k]) * 256 + threadIdx.x;
     if (k >= 3) {
         const int l = k - 3, i = (int)i0, N = U.N[l];
@@ -549,7 +549,7 @@ static cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int threads, size
 
 /* n products of one kind (n > 1: parts = 1) */
 template <int OPA, int OPB, int EPI>
-static cudaError_t gemm_tc(const GemmArgs* g, int n, int parts, cudaStream_t s) {
+static cudaError_t gemm_tc(const GemmArgs* g, int n, int parts, unsigned int* err, cudaStream_t s) {
     /* the weight gradients make two CTAs an SM of four K steps at a usual
      * batch; the rest one CTA of up to eight, all of them in flight at once */
     constexpr int S = EPI == EPI_GRAD ? 4 : 8;
@@ -559,6 +559,7 @@ static cudaError_t gemm_tc(const GemmArgs* g, int n, int parts, cudaStream_t s) 
     if (e != cudaSuccess) return e;
     GemmGroup P;
     memset(&P, 0, sizeof(P));
+    P.err = err;
     unsigned int tiles = 0;
     for (int i = 0; i < 3; i++) {
         P.first[i] = i < n ? tiles : 0xFFFFFFFFu;
@@ -601,6 +602,7 @@ struct vt_mlp {
     float* gw[3] = {}; float* gb[3] = {};
     float* mw[3] = {}; float* vw[3] = {}; float* mb[3] = {}; float* vb[3] = {};
     float* loss = nullptr;
+    unsigned int* err = nullptr;          /* device word: a bounded tensor-core wait of this network gave up */
     /* SIMT path: FP32 activations (act[0] = input copy) and gradients */
     float* act[4] = {};
     float* dact[4] = {};
@@ -614,13 +616,15 @@ struct vt_mlp {
     bool tc = true;                       /* GEMMs on the tensor cores (tcgen05); false: SIMT FMA */
 };
 
-/* a bounded tensor-core wait gave up (reported by the synchronising calls) */
-static vt_status mma_status() {
+/* A bounded tensor-core wait of this network gave up since the last report:
+ * reported by the calls that synchronise (a training step that returns its
+ * loss, gradients, reading and setting the weights); until then no training
+ * step changes the parameters. */
+static vt_status mma_status(vt_mlp* m) {
     unsigned int e = 0;
-    if (cudaMemcpyFromSymbol(&e, g_mma_err, sizeof(e)) != cudaSuccess) return vtrt::fail(VT_ERR_CUDA, "MLP status read");
+    if (cudaMemcpy(&e, m->err, sizeof(e), cudaMemcpyDeviceToHost) != cudaSuccess) return vtrt::fail(VT_ERR_CUDA, "MLP status read");
     if (e) {
-        e = 0;
-        cudaMemcpyToSymbol(g_mma_err, &e, sizeof(e));
+        cudaMemset(m->err, 0, sizeof(e));
         return vtrt::fail(VT_ERR_TIMEOUT, "a tensor-core GEMM did not complete within its wait bound");
     }
     return VT_OK;
@@ -710,7 +714,9 @@ extern "C" vt_status vt_mlp_create(int in, int h1, int h2, int out, uint64_t see
         }
         if (st != VT_OK) { vt_mlp_free(m); return st; }
     }
-    if (cudaMalloc(&m->loss, 4) != cudaSuccess) { vt_mlp_free(m); return vtrt::fail(VT_ERR_NOMEM, "MLP loss"); }
+    if (cudaMalloc(&m->loss, 8) != cudaSuccess) { vt_mlp_free(m); return vtrt::fail(VT_ERR_NOMEM, "MLP loss"); }
+    m->err = (unsigned int*)m->loss + 1;
+    if (cudaMemset(m->loss, 0, 8) != cudaSuccess) { vt_mlp_free(m); return vtrt::fail(VT_ERR_CUDA, "MLP init"); }
     *res = m;
     return VT_OK;
 }
@@ -740,15 +746,15 @@ static vt_status forward_tc(vt_mlp* m, const float* x, int batch, float* p, __nv
     g.Cb = h1; g.ldcb = m->ld[1]; g.C = y ? m->ha[1] : nullptr; g.ldc = d[1];
     g.loss = y ? m->loss : nullptr;   /* cleared */
     g.Xb = y ? m->xb : nullptr; g.ldx = m->ld[0];
-    CKM((gemm_tc<OP_F32_K, OP_BF16_MN, EPI_HIDDEN>(&g, 1, 1, s)));
+    CKM((gemm_tc<OP_F32_K, OP_BF16_MN, EPI_HIDDEN>(&g, 1, 1, m->err, s)));
     g.loss = nullptr;
     g.A = h1; g.lda = m->ld[1]; g.B = m->wb[1]; g.ldb = m->ld[2]; g.N = d[2]; g.K = g.kPer = d[1]; g.bias = m->b[1];
     g.Cb = h2; g.ldcb = m->ld[2]; g.C = y ? m->ha[2] : nullptr; g.ldc = d[2];
-    CKM((gemm_tc<OP_BF16_K, OP_BF16_MN, EPI_HIDDEN>(&g, 1, 1, s)));
+    CKM((gemm_tc<OP_BF16_K, OP_BF16_MN, EPI_HIDDEN>(&g, 1, 1, m->err, s)));
     g.A = h2; g.lda = m->ld[2]; g.B = m->wb[2]; g.ldb = m->ld[3]; g.N = d[3]; g.K = g.kPer = d[2]; g.bias = m->b[2];
     g.C = p; g.ldc = d[3];
     g.Y = y; g.invB = 1.0f / batch; g.loss = m->loss; g.Cb = m->dz[3]; g.ldcb = m->ld[3]; g.colsum = m->cs[3];
-    CKM((gemm_tc<OP_BF16_K, OP_BF16_MN, EPI_OUT>(&g, 1, 1, s)));
+    CKM((gemm_tc<OP_BF16_K, OP_BF16_MN, EPI_OUT>(&g, 1, 1, m->err, s)));
     return VT_OK;
 }
 
@@ -767,7 +773,7 @@ static vt_status train_tc(vt_mlp* m, const float* x, const float* y, int batch, 
         g.M = batch; g.N = d[l]; g.K = d[l + 1];
         g.C = m->part;
         const int parts = k_parts(g.M, g.N, g.K, &g.kPer);
-        CKM((gemm_tc<OP_BF16_K, OP_BF16_K, EPI_PART>(&g, 1, parts, s)));
+        CKM((gemm_tc<OP_BF16_K, OP_BF16_K, EPI_PART>(&g, 1, parts, m->err, s)));
         CKM(launch_pdl(k_dgrad_finish, dim3(((unsigned int)d[l] + 63) / 64 * (((unsigned int)batch + 15) / 16)), 256, 0, s,
                        m->part, parts, m->ha[l], batch, d[l], m->dz[l], m->ld[l], m->cs[l]));
     }
@@ -781,7 +787,7 @@ static vt_status train_tc(vt_mlp* m, const float* x, const float* y, int batch, 
         g[i].M = d[l]; g[i].N = d[l + 1]; g[i].K = g[i].kPer = batch;
         g[i].C = m->gw[l]; g[i].ldc = d[l + 1];
     }
-    CKM((gemm_tc<OP_BF16_MN, OP_BF16_MN, EPI_GRAD>(g, 3, 1, s)));
+    CKM((gemm_tc<OP_BF16_MN, OP_BF16_MN, EPI_GRAD>(g, 3, 1, m->err, s)));
     for (int l = 0; l < 3; l++) {
         u.w[l] = m->w[l]; u.m[l] = m->mw[l]; u.v[l] = m->vw[l]; u.g[l] = m->gw[l]; u.wb[l] = m->wb[l];
         u.rows[l] = d[l]; u.N[l] = d[l + 1]; u.ldb[l] = m->ld[l + 1];
@@ -795,6 +801,7 @@ static vt_status train_tc(vt_mlp* m, const float* x, const float* y, int batch, 
         blocks += (unsigned int)(d[l + 1] + 255) / 256;
     }
     if (adam) { u.adam = *adam; u.step = 1; }
+    u.err = m->err;
     CKM(launch_pdl(k_update, dim3(blocks), 256, 0, s, u));
     return VT_OK;
 }
@@ -872,7 +879,7 @@ extern "C" vt_status vt_mlp_train_step(vt_mlp* m, const float* dev_x, const floa
     if (loss) {
         CKM(cudaMemcpyAsync(loss, m->loss, 4, cudaMemcpyDeviceToHost, s));
         CKM(cudaStreamSynchronize(s));
-        return mma_status();
+        return mma_status(m);
     }
     return VT_OK;
 }
@@ -898,7 +905,16 @@ extern "C" vt_status vt_mlp_gradients(vt_mlp* m, const float* dev_x, const float
         CKM(cudaMemcpy(host_grads + o, m->gb[l], (size_t)m->dims[l + 1] * 4, cudaMemcpyDeviceToHost)); o += m->dims[l + 1];
     }
     if (loss) CKM(cudaMemcpy(loss, m->loss, 4, cudaMemcpyDeviceToHost));
-    return mma_status();
+    return mma_status(m);
+}
+
+extern "C" vt_status vt_debug_mlp_timeout(vt_mlp* m) {
+    vtrt::clear_error();
+    if (!m) return vtrt::fail(VT_ERR_INVALID, "null argument");
+    const unsigned int e = 1;
+    CKM(cudaDeviceSynchronize());
+    CKM(cudaMemcpy(m->err, &e, sizeof(e), cudaMemcpyHostToDevice));
+    return VT_OK;
 }
 
 extern "C" vt_status vt_mlp_use_tensor_cores(vt_mlp* m, int on) {
@@ -926,6 +942,8 @@ extern "C" vt_status vt_mlp_get_weights(vt_mlp* m, float* host, int64_t* n) {
     if (!host) return VT_OK;
     if (cap < total) return vtrt::fail(VT_ERR_INVALID, "need %lld floats", (long long)total);
     CKM(cudaDeviceSynchronize());
+    const vt_status st = mma_status(m);
+    if (st != VT_OK) return st;
     size_t o = 0;
     for (int l = 0; l < 3; l++) {
         size_t nw = (size_t)m->dims[l] * m->dims[l + 1];
@@ -949,7 +967,7 @@ extern "C" vt_status vt_mlp_set_weights(vt_mlp* m, const float* host, int64_t n)
         k_to_bf16<<<g1((long long)nw), 256>>>(m->w[l], m->wb[l], (long long)nw, m->dims[l + 1], m->ld[l + 1]);
     }
     CKM(cudaDeviceSynchronize());
-    return VT_OK;
+    return mma_status(m);
 }
 
 /* ------------------------------------------------------------------------ */
