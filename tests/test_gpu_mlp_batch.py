@@ -34,3 +34,25 @@ def test_large_training_batch(batch, cuda):
         for a0, a1, gg in ((w0, w1, gw), (b0, b1, gb)):
             want = a0 - 1e-2 * gg / (np.abs(gg) + 1e-8)
             assert np.abs(a1 - want).max() <= 1e-5 * (1 + np.abs(a0).max())
+
+
+def test_narrow_network_over_many_rows(cuda):
+    """A forward pass of 4-8-8-8 over 2^20 rows: 830 us with the kernel that
+    staged one K step at a time, 1025 where every CTA takes the shared memory
+    of eight whatever K is, and so an SM to itself."""
+    torch, batch = cuda, 1 << 20
+    m = vt.MLP((4, 8, 8, 8), seed=4)
+    x, p = torch.randn(batch, 4, device="cuda"), torch.empty(batch, 8, device="cuda")
+    us = []
+    for _ in range(6):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        m.forward(x, batch, p)
+        b.record()
+        torch.cuda.synchronize()
+        us.append(a.elapsed_time(b) * 1e3)
+    assert min(us) < 830
+    # and the last rows are those of the same rows alone
+    q = torch.empty(100, 8, device="cuda")
+    m.forward(x[-100:].contiguous(), 100, q)
+    assert torch.equal(p[-100:], q)

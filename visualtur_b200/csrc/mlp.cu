@@ -18,6 +18,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -561,13 +562,19 @@ static cudaError_t gemm_tc(const GemmArgs* g, int n, int parts, unsigned int* er
     memset(&P, 0, sizeof(P));
     P.err = err;
     unsigned int tiles = 0;
+    int stages = 0;
     for (int i = 0; i < 3; i++) {
         P.first[i] = i < n ? tiles : 0xFFFFFFFFu;
         if (i >= n) continue;
         P.g[i] = g[i];
+        stages = std::max(stages, (g[i].kPer + G_K - 1) / G_K);
         tiles += (unsigned int)((g[i].N + G_N - 1) / G_N) * (unsigned int)((g[i].M + G_M - 1) / G_M);
     }
-    return launch_pdl(k_gemm_tc<OPA, OPB, EPI, S>, dim3(tiles, 1, parts), G_THREADS, S * G_STAGE_BYTES, s, P);
+    /* a product of fewer K steps uses as many stages: with a narrow network
+     * and a large batch several CTAs then share an SM (4-8-8-8, 1 048 576
+     * rows: 1025 -> 340 us a forward pass) */
+    const size_t smem = std::max((size_t)std::min(stages, S) * G_STAGE_BYTES, (size_t)G_M * (G_N + 1) * 4);
+    return launch_pdl(k_gemm_tc<OPA, OPB, EPI, S>, dim3(tiles, 1, parts), G_THREADS, smem, s, P);
 }
 /* K parts of a product with few tiles: enough to give every SM one, each at
  * least two K steps deep */
