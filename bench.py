@@ -110,7 +110,7 @@ CONFIGS = {
 
 # renderer modes: "plain" = the reference's scheme (one view per launch,
 # demand LRU from a cold cache, no prefetch); "best" = the product: batches
-# of 8 frames per persistent ray-queue launch, lookahead requests, learned
+# of 8 frames per launch, lookahead requests, learned
 # prefetch hints for the next batch, kernel knobs from the autotuner
 MODES = {
     "plain": dict(opts=dict(persistent=0, lookahead=0, use_graph=0), batch=1, learned=False, autotune=False),
@@ -995,7 +995,7 @@ def tune_paging(wl, cfg, torch, dev, stream, P, f0, frames=96):
 
 
 def autotune(args, wl, cfg, torch, dev, stream, frame0, batch):
-    """Kernel schedule sweep (tile x unroll x persistent) on the renderer;
+    """Kernel schedule sweep (tile x unroll) on the renderer;
     for the batched workload first the brick edge {8, 16, 32} at the
     default schedule, keeping the fastest renderer."""
     from visualtur_b200 import autotune as at

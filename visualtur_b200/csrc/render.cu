@@ -5,17 +5,20 @@
  * traversal (cuda_getFirtsVoxel, src/Octree.cu:620-739), cache lookup
  * (lruCache::updateCube, src/lruCache.cu:168-296) and march + shade
  * (cuda_rayCaster, src/rayCaster.cu:139-265) -- into one kernel: each ray
- * walks its DFS, marches every candidate node whose brick is resident, and
- * either finishes or suspends with its stack saved when a brick is absent.
- * The result equals the reference's iterate-until-PAINTED loop: candidates
- * are marched in the same DFS order and the first hit is shaded.  The
- * instantiations with SKIP = true let a ray set absent-brick candidates
- * aside and march later ones in the same pass (see run_ray); the first hit
- * in DFS order still decides the pixel.
+ * walks from candidate node to candidate node, marches every one whose brick
+ * is resident, and either finishes or, at an absent brick, suspends with the
+ * cell it has come to.  The result equals the reference's
+ * iterate-until-PAINTED loop: candidates are marched in its depth-first
+ * order and the first hit is shaded.  The instantiations with SKIP = true
+ * let a ray set absent-brick candidates aside and march later ones in the
+ * same pass (see run_ray); the first hit in that order still decides the
+ * pixel.
  *
- * Octree: a flattened node array with 8-bit child masks holding the result
- * of the reference's range search (computed once per octree load), and the
- * same tree two levels at a time (tree64.cuh), which k_trace walks.
+ * Octree: the same tree twice, from a flattened node array with 8-bit child
+ * masks that hold the result of the reference's range search (computed once
+ * per octree load).  k_trace walks it two levels at a time (tree64.cuh);
+ * rays that meet coinciding planes, and the wavefront passes, search the
+ * binary nodes depth first and suspend with their stack.
  */
 #include "vt_kernels.h"
 #include "vt_math.cuh"
@@ -476,11 +479,10 @@ __device__ __forceinline__ int candidate(const TraceArgs& A, Ray& R, unsigned lo
     return CAND_HIT;
 }
 
-/* Advances one ray's DFS by at most `budget` steps (src/Octree.cu:620-720
- * interleaved with src/rayCaster.cu:139-265): inner nodes are expanded
- * until a candidate is on top, then the candidate is marched.  Returns
- * RAY_DONE when the ray is shaded or exhausted, RAY_SUSPENDED when it must
- * wait for absent bricks, RAY_RUNNING when the budget ran out.
+/* Takes one ray's DFS to its end (src/Octree.cu:620-720 interleaved with
+ * src/rayCaster.cu:139-265): inner nodes are expanded until a candidate is
+ * on top, then the candidate is marched.  Returns RAY_DONE when the ray is
+ * shaded or exhausted, RAY_SUSPENDED when it must wait for absent bricks.
  *
  * Passing over absent bricks (A.ctl.skip > 0): a candidate whose brick is
  * absent is requested and set aside, and the DFS goes on to later
@@ -492,7 +494,7 @@ __device__ __forceinline__ int candidate(const TraceArgs& A, Ray& R, unsigned lo
  * in several absent bricks asks for all of them in one pass instead of one
  * per pass, and the image is the one of the in-order traversal. */
 template <int VTYPE, bool SLAB, int U, bool SKIP>
-__device__ int run_ray(const TraceArgs& A, Ray& R, Stk& st, unsigned int* cnt, int budget) {
+__device__ int run_ray(const TraceArgs& A, Ray& R, Stk& st, unsigned int* cnt) {
     const int Lo = A.oct.Lo;
     if (SKIP) {
         while (R.resumeSkips) {
@@ -501,7 +503,6 @@ __device__ int run_ray(const TraceArgs& A, Ray& R, Stk& st, unsigned int* cnt, i
                 if (R.tent) return RAY_DONE_WRITTEN;
                 break;
             }
-            if (budget-- == 0) return RAY_RUNNING;
             const int c = candidate<VTYPE, SLAB, U>(A, R, st.sk[0], cnt);
             if (c == CAND_MISSING) return RAY_SUSPENDED;
             for (int k = 1; k < R.nskip; k++) st.sk[k - 1] = st.sk[k];
@@ -516,12 +517,10 @@ __device__ int run_ray(const TraceArgs& A, Ray& R, Stk& st, unsigned int* cnt, i
             if (R.top < 0) return (SKIP && R.nskip > 0) ? RAY_SUSPENDED : RAY_DONE;   /* exhausted: background */
             ent = st.e[R.top];
             if (e_level(ent) == Lo) break;
-            if (budget-- == 0) return RAY_RUNNING;
             R.top--;
             cnt[VT_C_EXPANSIONS]++;
             if (!expand(A, R.r, st, R.top, ent, cnt, true)) return RAY_DONE;
         }
-        if (budget-- == 0) return RAY_RUNNING;
         if (R.taken) { R.taken--; R.top--; continue; }
         const int c = candidate<VTYPE, SLAB, U>(A, R, ent, cnt);
         if (c == CAND_MISSING) {
@@ -695,7 +694,7 @@ __device__ __forceinline__ void search_ray(const TraceArgs& A, const DevView* sv
         R.nskip = nskip;
         for (int e = 0; e < nskip; e++) st.sk[e] = sk[e];
     }
-    if (s == RAY_RUNNING) s = run_ray<VTYPE, SLAB, U, SKIP>(A, R, st, cnt, -1);
+    if (s == RAY_RUNNING) s = run_ray<VTYPE, SLAB, U, SKIP>(A, R, st, cnt);
     if (s == RAY_DONE) write_ray(A, sv, R, cnt);
     else if (SKIP && s == RAY_TENTATIVE) {
         write_ray(A, sv, R, cnt, false);
@@ -1432,8 +1431,11 @@ cudaError_t vt_launch_trace(const TraceArgs& a0, bool slabMode, cudaStream_t s) 
     TraceArgs a = a0;
     /* a full warp a tile, unless that leaves the GPU short of warps: then
      * fewer rays a warp, which diverge less.  A warp's time is the sum of its
-     * lanes' separate turns, so on a 96x96 frame (288 full warps for 4144
-     * places) 32, 16, 8, 4, 1 rays a warp took 74, 61, 50, 49, 45 us. */
+     * lanes' separate turns, so on a 96x96 frame (288 full warps for 3552
+     * places) pass 0 took 74, 75, 70, 68, 63, 62 us with 32, 16, 8, 4, 2, 1
+     * rays a warp; the rule takes 2 there.  Later passes have no more rays
+     * than earlier ones, so records of k_trace's walk never come to
+     * k_literal, which reads saved stacks only. */
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

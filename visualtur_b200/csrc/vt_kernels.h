@@ -95,8 +95,7 @@ struct DevViews {
 };
 
 /* A suspended ray: padded global ray index, saved stack depth (0 = restart
- * from the root) and offset of its entries in the stack pool. */
-/* A suspended ray: its pool entries at `off` are its passed-over
+ * from the root) and offset of its entries in the stack pool.  Its pool entries at `off` are its passed-over
  * candidates (depth bits 8-10), then its DFS stack (bits 0-7); bit 11: its
  * pixel already holds a hit found past those candidates; bit 12: instead of
  * a stack the entry is the candidate the 64-ary walk stopped at, and bits
@@ -109,7 +108,7 @@ struct SuspRec {
     unsigned long long off;
 };
 
-/* Per-pass control: counters, error bits, work queue, demand paging. */
+/* Per-pass control: counters, error bits, rays to resume, demand paging. */
 struct DevCtl {
     unsigned long long* counters;
     unsigned int* err;
@@ -159,9 +158,6 @@ struct MarchItem {
     unsigned int pad;
 };
 struct WaveRound {
-    /* input of this round: the pass's rays (in == NULL in a first pass: ray
-     * indices 0..count) or the previous round's waiting records */
-    const SuspRec* in; const unsigned int* n_in; unsigned int n_in_host; const unsigned long long* pool_in;
     /* waiting rays of this round */
     SuspRec* wait; unsigned int* n_wait; unsigned long long* pool_wait; unsigned long long* pool_wait_used;
     unsigned long long pool_wait_cap; unsigned int wait_cap;
@@ -170,8 +166,6 @@ struct WaveRound {
     unsigned int* binCount; unsigned int* binStart; unsigned int* touched; unsigned int* n_touched;
     /* rays whose candidate missed: the next round's input */
     SuspRec* next; unsigned int* n_next;
-    unsigned int* work;         /* persistent work counter */
-    int last;                   /* last round: misses join the pass's suspended list instead */
 };
 
 /* launchers (render.cu) */
