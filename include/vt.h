@@ -128,7 +128,9 @@ vt_status vt_octree_info(const vt_octree* o, float* iso, int* dimension, int rea
 /* Number of uint64 words of level `level` and a copy of them. */
 vt_status vt_octree_level(const vt_octree* o, int level, int64_t* n, uint64_t* words);
 /* OctreeM::OctreeM + writeToFile (src/CreateOctree.cu:300-371) on the GPU:
- * builds the octree of `v` for isovalue `iso` and writes the file. */
+ * builds the octree of `v` for isovalue `iso` and writes the file.  A regular
+ * file at out_path is replaced when the new one is whole: a build that fails
+ * on the device leaves it as it was. */
 vt_status vt_octree_build(const vt_volume* v, float iso, const char* out_path, void* stream);
 /* Same for a volume already in device memory (dims[0]*dims[1]*dims[2]
  * voxels of vtype, x slowest). */

@@ -105,3 +105,30 @@ def test_lattice_camera_parity(pos, mode, edge, workdir, cuda):
     assert st["rays"] == edge * edge and st["hits"] == want["agg"]["hits"] > 0
     if mode != "cold_skip":
         assert st["samples"] == want["agg"]["samples"] and st["candidates"] == want["agg"]["candidates"]
+
+
+def test_cameras_on_and_off_the_lattice_through_one_graph(scenes, cuda):
+    """Pass 0 is a captured graph whose kernel changes with the camera."""
+    torch = cuda
+    fm, oc, brick = scenes["blobs"]
+    lc = oc.nLevels - 4
+    p = vt.make_params(W=640, H=480, octreeFile=None, hdf5File=None, octreeLevel=oc.nLevels - 2, levelCubes=lc,
+                       dimCube=brick, maxElementsCache=8 ** lc, maxElementsCache_CPU=8 ** lc)
+    cams = [look_at(640, 480, 50.0, 30.0, np.array(pos, float), np.array((168.0, 188.0, 218.0)))
+            for pos in (INSIDE, LATTICE, LATTICE, INSIDE, (256, 256, 256), INSIDE)]
+    images = []
+    for graph in (0, 1):
+        r = vt.visualTur(p, vt.default_options(preload=1, skip=0, lookahead=0, use_graph=graph), volume=fm, octree=oc)
+        s, out = torch.cuda.Stream(), []
+        for c in cams:
+            r.set_camera(c)
+            rgba = torch.empty(640 * 480, 4, device="cuda")
+            torch.cuda.synchronize()
+            r.updateVisibleCubes(rgba, stream=s.cuda_stream)
+            s.synchronize()
+            out.append(rgba)
+        images.append(out)
+        r.close()
+    for a, b in zip(*images):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    assert not torch.equal(images[0][0], images[0][1])
