@@ -77,6 +77,35 @@ def test_camera_on_a_lattice_point_costs_no_more_than_the_binary_search(name, mo
     assert trace_ms(scenes[name], LATTICE) < most * trace_ms(scenes[name], INSIDE)
 
 
+@pytest.mark.parametrize("mode", ["resident", "slab", "cold", "cold_skip"])
+@pytest.mark.parametrize("pos, fov, edge", [((64, 64, 200), 45.0, 200), ((64, 64, 200), 45.0, 201), ((63, 61, 160), 45.0, 128),
+                                            ((128, 128, 192), 45.0, 160)])
+def test_late_coincidences_parity(pos, fov, edge, mode, workdir, cuda):
+    """Cameras on lattice points outside with a pixel grid of round numbers,
+    against the oracle: the image, and (in order) every candidate once."""
+    c = F.CASES["c1"]
+    vol, path = F.case_volume("c1"), F.case_octree("c1", workdir)
+    nb = 8 ** c["levelC"] if not mode.startswith("cold") else 40
+    p = vt.make_params(W=edge, H=edge, octreeFile=None, hdf5File=None, octreeLevel=c["levelO"], levelCubes=c["levelC"],
+                       dimCube=8, cubeInc=c["inc"], distance=c["dist"], fov_H=fov, fov_W=fov,
+                       maxElementsCache=nb, maxElementsCache_CPU=nb)
+    opt = vt.default_options(resident=mode == "resident", preload=0, record_hits=1, lookahead=0, max_passes=100000,
+                             skip=2 if mode == "cold_skip" else 0)
+    r = vt.visualTur(p, opt, volume=vt.FileManager.wrap(vol), octree=vt.Octree(path))
+    r.camera_Move(pos)
+    rgba, rgb8 = r.render_host()
+    node, brick, t, nrm = r.debug_hits()
+    st = r.stats()
+    r.close()
+    cam = orc.Camera(edge, edge, c["dist"], fov, fov)
+    orc.apply_ops(cam, [("mv", pos)])
+    want = orc.render(orc.Octree(path), vol, cam, c["levelO"], c["levelC"], c["inc"])
+    assert_parity(dict(rgba=rgba, rgb8=rgb8, node=node, brick=brick, t=t, normal=nrm), want)
+    assert st["hits"] == want["agg"]["hits"] > 0
+    if mode != "cold_skip":
+        assert st["samples"] == want["agg"]["samples"] and st["candidates"] == want["agg"]["candidates"]
+
+
 @pytest.mark.parametrize("edge", [64, 384])     # few rays a warp, full warps (the search's own kernel)
 @pytest.mark.parametrize("mode", ["resident", "slab", "cold", "cold_skip", "wave"])
 @pytest.mark.parametrize("pos", [(64, 64, 64), (32, 60.5, 64), (64, 44, 128)])
