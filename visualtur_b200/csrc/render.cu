@@ -681,15 +681,14 @@ __device__ __forceinline__ void flush_counters(const TraceArgs& A, unsigned int*
 }
 
 /* The literal depth-first search for one ray, to its end.  sk: set-aside
- * candidates of a ray handed over by the walk. */
+ * candidates of a ray handed over by the walk.  False for tile padding. */
 template <int VTYPE, bool SLAB, int U, bool SKIP>
-__device__ __forceinline__ void search_ray(const TraceArgs& A, const DevView* sv, const SuspRec& rec, int nskip,
+__device__ __forceinline__ bool search_ray(const TraceArgs& A, const DevView* sv, const SuspRec& rec, int nskip,
                                            const unsigned long long* sk, unsigned int* cnt) {
     Stk st;
     Ray R;
     int s = start_ray<SKIP>(A, sv, rec, R, st);
-    if (s < 0) return;
-    if (!A.ctl.in && !rec.depth) cnt[VT_C_RAYS]++;
+    if (s < 0) return false;
     if (SKIP && nskip > 0) {
         R.nskip = nskip;
         for (int e = 0; e < nskip; e++) st.sk[e] = sk[e];
@@ -701,6 +700,7 @@ __device__ __forceinline__ void search_ray(const TraceArgs& A, const DevView* sv
         suspend_ray<VTYPE, SLAB, SKIP>(A, R, st, cnt);
     } else if (s == RAY_SUSPENDED) suspend_ray<VTYPE, SLAB, SKIP>(A, R, st, cnt);
     else if (SKIP && s == RAY_DONE_WRITTEN) cnt[VT_C_HITS]++;   /* the tentative hit stands */
+    return true;
 }
 
 /* The literal search in k_trace: rays whose 64-ary walk met coinciding or
@@ -1028,7 +1028,7 @@ __global__ void __launch_bounds__(128, 8) k_literal(const __grid_constant__ Trac
         SuspRec rec;
         if (A.ctl.in) rec = A.ctl.in[w];
         else { rec.ray = w; rec.depth = 0; }
-        search_ray<VTYPE, SLAB, 1, SKIP>(A, A.views.v, rec, 0, nullptr, cnt);
+        if (search_ray<VTYPE, SLAB, 1, SKIP>(A, A.views.v, rec, 0, nullptr, cnt) && !A.ctl.in) cnt[VT_C_RAYS]++;
     }
     __syncwarp();
     flush_counters(A, cnt);
